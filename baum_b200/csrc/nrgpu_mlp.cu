@@ -300,87 +300,123 @@ __global__ void refresh_bf16_kernel(const float *__restrict__ P, __nv_bfloat16 *
 }
 
 // ---- FP32 inference (CUDA cores) ------------------------------------------------
-// The whole forward pass for 32 grid points per block, in FP32 from the FP32
+// The whole forward pass for 128 grid points per block, in FP32 from the FP32
 // master weights: features rounded to FP32 only (not BF16), hidden products
-// as a 32 x 128 x K register-tiled SIMT product (thread: 2 rows x 8
-// columns), bias + SiLU, the output layer by a warp reduction; u = s out.
+// as a 128 x 128 x K register-tiled product (thread: 8 rows x 8 columns),
+// bias + SiLU, the output layer by a warp reduction; u = s out.
 // Used to evaluate the trained network without the BF16 rounding of the
 // training path (whose grid-scale noise the undamped Jacobi smoother of the
 // multigrid does not remove).
-constexpr int kFR = 32;   // rows (grid points) per block
-__global__ void __launch_bounds__(256) mlp_forward_fp32_kernel(const double *__restrict__ cond, int m, double dx,
-                                                               const float *__restrict__ P, double s, double *u,
-                                                               long np) {
-  __shared__ float act[2][kFR][HID];
+// Bound by the FP32 units.  The activations stay in shared memory with the
+// rows of one feature side by side, the weights pass through it in chunks of
+// 16 features fetched ahead by cp.async: 4 16-byte loads per 64 FMAs and
+// thread.  Two blocks per SM, so that one's SiLU runs beside the other's FMAs.
+constexpr int kFR = 128;          // rows (grid points) per block
+constexpr int kFP = kFR + 4;      // row pitch: 8 lanes' 16-byte stores at stride kFP meet no bank twice
+constexpr int kFK = 16;           // features per weight chunk
+constexpr int kFSmem = (HID * kFP + 2 * kFK * HID) * (int)sizeof(float);
+
+// chunk c of a layer's weights into buf: column cg + 16 q of a feature at
+// (q / 4) 64 + 4 cg + q % 4, i.e. a thread's 8 columns as two 16-byte words
+__device__ __forceinline__ void weights_ahead(float *buf, const float *__restrict__ W, int c, int t) {
+#pragma unroll
+  for (int e = t; e < kFK * HID; e += 256) {
+    const int k = e / HID, j = e % HID, q = j / 16;
+    const unsigned d = (unsigned)__cvta_generic_to_shared(buf + k * HID + (q / 4) * 64 + (j % 16) * 4 + q % 4);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(W + (long)c * kFK * HID + e) : "memory");
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+__global__ void __launch_bounds__(256, 2) mlp_forward_fp32_kernel(const double *__restrict__ cond, int m, double dx,
+                                                                  const float *__restrict__ P, double s, double *u,
+                                                                  long np) {
+  extern __shared__ __align__(16) float fsm[];
+  float *act = fsm, *wb = fsm + HID * kFP;  // act[feature][row], two weight chunks
   const int t = threadIdx.x;
   const long first = (long)blockIdx.x * kFR;
+  weights_ahead(wb, P + off_w(0), 0, t);
   // features of the block's rows (the formulas of mlp_features_kernel)
   if (t < kFR) {
-    float *f = act[0][t];
+    float *f = act + t;
     const long p = min(first + t, np - 1);
     const double h0 = -0.5 * (m - 1) * dx;
     const int i = (int)(p % m), j = (int)((p / m) % m), k = (int)(p / ((long)m * m));
     const double x[3] = {h0 + i * dx, h0 + j * dx, h0 + k * dx};
     const double sc = 1.0 / 8.0;
     f[0] = (float)(x[0] * sc);
-    f[1] = (float)(x[1] * sc);
-    f[2] = (float)(x[2] * sc);
+    f[kFP] = (float)(x[1] * sc);
+    f[2 * kFP] = (float)(x[2] * sc);
     for (int q = 0; q < 2; ++q) {
       const double mq = cond[q];
       const double d0 = x[0] - cond[2 + 3 * q], d1 = x[1] - cond[3 + 3 * q], d2 = x[2] - cond[4 + 3 * q];
       const double rr = sqrt(d0 * d0 + d1 * d1 + d2 * d2);
-      float *g = f + 3 + 12 * q;
+      float *g = f + (3 + 12 * q) * kFP;
       g[0] = (float)(d0 * sc);
-      g[1] = (float)(d1 * sc);
-      g[2] = (float)(d2 * sc);
-      g[3] = (float)(rr * sc);
-      g[4] = (float)(mq / (rr + mq));
-      g[5] = (float)(2.0 * mq);
+      g[kFP] = (float)(d1 * sc);
+      g[2 * kFP] = (float)(d2 * sc);
+      g[3 * kFP] = (float)(rr * sc);
+      g[4 * kFP] = (float)(mq / (rr + mq));
+      g[5 * kFP] = (float)(2.0 * mq);
       for (int a = 0; a < 3; ++a) {
-        g[6 + a] = (float)(5.0 * cond[8 + 3 * q + a]);
-        g[9 + a] = (float)(5.0 * cond[14 + 3 * q + a]);
+        g[(6 + a) * kFP] = (float)(5.0 * cond[8 + 3 * q + a]);
+        g[(9 + a) * kFP] = (float)(5.0 * cond[14 + 3 * q + a]);
       }
     }
-    for (int q = 27; q < IN; ++q) f[q] = 0.0f;
+    for (int q = 27; q < IN; ++q) f[q * kFP] = 0.0f;
+  }
+  const int cg = t % 16, rg = t / 16;  // columns cg + 16 q, rows 4 rg .. 4 rg + 3 and 64 further
+  int buf = 0;
+  for (int l = 0; l < 4; ++l) {
+    const int nc = fan_in(l) / kFK;
+    const float *W = P + off_w(l), *bias = P + off_b(l);
+    float acc[8][8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+#pragma unroll
+      for (int q = 0; q < 8; ++q) acc[r][q] = 0.0f;
+    for (int c = 0; c < nc; ++c) {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncthreads();  // the chunk, and the layer's activations, are there; the other buffer is free
+      if (c + 1 < nc) weights_ahead(wb + (buf ^ 1) * kFK * HID, W, c + 1, t);
+      else if (l < 3) weights_ahead(wb + (buf ^ 1) * kFK * HID, P + off_w(l + 1), 0, t);
+      const float *wk = wb + buf * kFK * HID + 4 * cg, *ak = act + c * kFK * kFP + 4 * rg;
+#pragma unroll
+      for (int k = 0; k < kFK; ++k) {
+        float a[8], w[8];
+        *(float4 *)a = *(const float4 *)(ak + k * kFP);
+        *(float4 *)(a + 4) = *(const float4 *)(ak + k * kFP + 64);
+        *(float4 *)w = *(const float4 *)(wk + k * HID);
+        *(float4 *)(w + 4) = *(const float4 *)(wk + k * HID + 64);
+#pragma unroll
+        for (int r = 0; r < 8; ++r)
+#pragma unroll
+          for (int q = 0; q < 8; ++q) acc[r][q] = fmaf(a[r], w[q], acc[r][q]);
+      }
+      buf ^= 1;
+    }
+    __syncthreads();  // every thread has read the layer's input
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int col = cg + 16 * q;
+      const float bq = __ldg(bias + col);
+      float y[8];
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        const float z = acc[r][q] + bq;
+        y[r] = z * sigm(z);
+      }
+      *(float4 *)(act + col * kFP + 4 * rg) = *(float4 *)y;
+      *(float4 *)(act + col * kFP + 64 + 4 * rg) = *(float4 *)(y + 4);
+    }
   }
   __syncthreads();
-  const int cg = t % 16, rg = t / 16;   // columns 8 cg .. 8 cg + 7, rows 2 rg, 2 rg + 1
-  int cur = 0;
-  for (int l = 0; l < 4; ++l) {
-    const int K = fan_in(l);
-    const float *W = P + off_w(l), *bias = P + off_b(l);
-    float acc[2][8];
-#pragma unroll
-    for (int r = 0; r < 2; ++r)
-#pragma unroll
-      for (int c = 0; c < 8; ++c) acc[r][c] = 0.0f;
-    for (int k = 0; k < K; ++k) {
-      float w[8], a[2];
-#pragma unroll
-      for (int c = 0; c < 8; ++c) w[c] = __ldg(W + (long)k * HID + 8 * cg + c);
-#pragma unroll
-      for (int r = 0; r < 2; ++r) a[r] = act[cur][2 * rg + r][k];
-#pragma unroll
-      for (int r = 0; r < 2; ++r)
-#pragma unroll
-        for (int c = 0; c < 8; ++c) acc[r][c] = fmaf(a[r], w[c], acc[r][c]);
-    }
-#pragma unroll
-    for (int r = 0; r < 2; ++r)
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        const float z = acc[r][c] + __ldg(bias + 8 * cg + c);
-        act[cur ^ 1][2 * rg + r][8 * cg + c] = z * sigm(z);
-      }
-    __syncthreads();
-    cur ^= 1;
-  }
-  // out = A4 w5 + b5: warp w reduces rows 4 w .. 4 w + 3
+  // out = A4 w5 + b5: warp w reduces rows 16 w .. 16 w + 15
   const int w = t >> 5, lane = t & 31;
   const float *w5 = P + kOffW5;
-  for (int r = 4 * w; r < 4 * w + 4; ++r) {
+  for (int r = 16 * w; r < 16 * w + 16; ++r) {
     float v = 0.0f;
-    for (int k = lane; k < HID; k += 32) v = fmaf(act[cur][r][k], __ldg(w5 + k), v);
+    for (int k = lane; k < HID; k += 32) v = fmaf(act[k * kFP + r], __ldg(w5 + k), v);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
     if (lane == 0 && first + r < np) u[first + r] = s * (double)(v + __ldg(w5 + HID));
@@ -945,7 +981,8 @@ extern "C" int nrgpu_mlp_predict_u_fp32(nrgpu_mlp *M, const double *host_cond, i
   int e = set_cond(M, host_cond, 1);
   if (e) return e;
   const long np = (long)m * m * m;
-  mlp_forward_fp32_kernel<<<(unsigned)((np + kFR - 1) / kFR), 256, 0, st>>>(M->cond, m, dx, M->P, uscale, u, np);
+  NRGPU_CUDA_TRY(cudaFuncSetAttribute(mlp_forward_fp32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFSmem));
+  mlp_forward_fp32_kernel<<<(unsigned)((np + kFR - 1) / kFR), 256, kFSmem, st>>>(M->cond, m, dx, M->P, uscale, u, np);
   NRGPU_CUDA_TRY(cudaGetLastError());
   return NRGPU_OK;
 }
