@@ -10,14 +10,10 @@
 // reverse-mode chain with the same BF16 operands as the forward pass.
 //
 // Kernels:
-//   mlp_features_kernel   feature rows (double math, rounded to BF16)
-//   gemm_bf16_kernel      C[MxN] (+)= A[MxK] B[KxN], A/B stored plain or
-//                         transposed, split-K with FP32 atomics
-//   bias_silu_kernel      Z += b, A = bf16(silu(Z))
-//   out_layer_kernel      out = A4 w5 + b5; loss, dw5, db5, dZ4 (training)
-//   silu_back_kernel      dZ = bf16(dA * silu'(Z))
-//   colsum_kernel         db = sum over rows of dZ
-//   adam_kernel           Adam step on the FP32 master copy + BF16 refresh
+//   mlp_features_kernel     feature rows (double math, rounded to BF16)
+//   mlp_rows_kernel         forward, loss and backward of 128 rows per block
+//   mlp_weight_grad_kernel  dW = A^T dZ, split over row chunks with FP32 atomics
+//   adam_kernel             Adam step on the FP32 master copy + BF16 refresh
 #include <cuda_bf16.h>
 #include <stdint.h>
 #include <string.h>
@@ -80,204 +76,328 @@ __global__ void mlp_features_kernel(const double *__restrict__ cond, const int *
   for (int q = 27; q < IN; ++q) f[q] = __float2bfloat16_rn(0.0f);
 }
 
-// ---- BF16 GEMM on the tensor cores --------------------------------------------
-// C[M][N] (+)= A[M][K] B[K][N]; A stored [M][K] (AT = false) or [K][M] (AT =
-// true), B stored [K][N] (BT = false) or [N][K] (BT = true), all row major.
-// CTA tile 64 x 64, k step 32, 4 warps of 32 x 32.  M, N multiples of 16,
-// K of 32 (checked by the host).  ATOMIC: split-K over gridDim.z, the
-// caller zeroes C.
-constexpr int TM = 64, TN = 64, TK = 32, PADK = 40;
+// ---- forward and backward of 128 rows on the tensor cores -------------------------
+// One kernel runs the whole network over a block's 128 rows: the BF16 weights
+// of all layers lie in shared memory, two warps share 16 rows, each with half
+// of the columns of every layer, and pass their halves of the next operand
+// through shared memory (a barrier of the pair per layer); the backward pass
+// follows in the same way.  Training writes what the weight gradients need,
+// the BF16 activations and pre-activation gradients of every layer, and keeps
+// silu'(z) in FP32 (Z) between the passes.  With a kernel per product and per
+// elementwise step the same work took 32 launches and eleven passes over
+// 8 MB arrays: 380 us per step of 16384 rows.  What bounds it now is latency:
+// a step has rows for one block per SM, so 16 warps (with whole rows per
+// warp, 8 warps, this kernel took 100 us).
+constexpr int kWPitch = HID + 8;             // BF16 per weight row: ldmatrix meets no bank twice
+constexpr int kWRows = IN + 3 * HID;
+constexpr int kRowsSmem = (kWRows + 2 * 128) * kWPitch * 2;
 
-__device__ __forceinline__ void mma16816(float d[4], const uint32_t a[4], const uint32_t b[2]) {
+__device__ __forceinline__ float sigm(float z) { return 1.0f / (1.0f + expf(-z)); }
+
+__device__ __forceinline__ void mma16816(float d[4], const uint32_t a[4], uint32_t b0, uint32_t b1) {
   asm volatile(
       "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
       "{%0,%1,%2,%3};\n"
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void ldsm4(uint32_t r[4], const __nv_bfloat16 *p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"((unsigned)__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ void ldsm4t(uint32_t r[4], const __nv_bfloat16 *p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"((unsigned)__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ void cp16(void *dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t *>(&v);
+}
+__device__ __forceinline__ float2 unpack2(uint32_t v) {
+  return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&v));
 }
 
-// stage a 64 (outer) x 32 (k) tile into S[outer][k] from a row-major BF16
-// matrix: KCONTIG = the source rows run along k (S[o][k] = G[outer0+o][k0+k]),
-// otherwise along the outer index (S[o][k] = G[k0+k][outer0+o])
-template <bool KCONTIG>
-__device__ __forceinline__ void load_tile(__nv_bfloat16 (*S)[PADK], const __nv_bfloat16 *__restrict__ G, int ld,
-                                          int outer0, int nouter, int k0) {
-  const int t = threadIdx.x;
-  if (KCONTIG) {
-    const int o = t >> 1, kk = (t & 1) * 16;
-    uint4 v0 = make_uint4(0, 0, 0, 0), v1 = v0;
-    if (outer0 + o < nouter) {
-      const uint4 *src = reinterpret_cast<const uint4 *>(G + (long)(outer0 + o) * ld + k0 + kk);
-      v0 = __ldg(src);
-      v1 = __ldg(src + 1);
-    }
-    // rows of S are 80 bytes: 16-byte aligned at kk = 0 and 16
-    uint4 *dst = reinterpret_cast<uint4 *>(&S[o][kk]);
-    dst[0] = v0;
-    dst[1] = v1;
-  } else {
-    const int kk = t >> 2, o0 = (t & 3) * 16;
-    alignas(16) __nv_bfloat16 v[16];
-    if (outer0 + o0 < nouter) {
-      const uint4 *src = reinterpret_cast<const uint4 *>(G + (long)(k0 + kk) * ld + outer0 + o0);
-      *reinterpret_cast<uint4 *>(v) = __ldg(src);
-      *reinterpret_cast<uint4 *>(v + 8) = __ldg(src + 1);
-    } else {
-      for (int q = 0; q < 16; ++q) v[q] = __float2bfloat16_rn(0.0f);
-    }
+struct RowsArgs {
+  const __nv_bfloat16 *X, *Wb;  // features, weights of W1..W4
+  const float *P, *y;
+  float *out;                   // network output per row
+  float *Z[4];                  // silu'(z) (training)
+  __nv_bfloat16 *A[4], *dZ[4];  // activations, pre-activation gradients (training)
+  float *grad, *loss;
+  int n;
+};
+
+// sum over the rows of a warp's 16 x 8 tiles: v[0], v[1] = this thread's
+// columns 2 tg, 2 tg + 1; the lanes of row 0 add the result
+__device__ __forceinline__ void add_columns(float *dst, float v0, float v1, int lane) {
 #pragma unroll
-    for (int q = 0; q < 16; ++q) S[o0 + q][kk] = v[q];
+  for (int o = 4; o < 32; o <<= 1) {
+    v0 += __shfl_xor_sync(0xffffffffu, v0, o);
+    v1 += __shfl_xor_sync(0xffffffffu, v1, o);
+  }
+  if (lane < 4) {
+    atomicAdd(dst + 2 * lane, v0);
+    atomicAdd(dst + 2 * lane + 1, v1);
   }
 }
 
-template <bool AT, bool BT, bool ATOMIC>
-__global__ void __launch_bounds__(128) gemm_bf16_kernel(const __nv_bfloat16 *__restrict__ A,
-                                                        const __nv_bfloat16 *__restrict__ B, float *C, int M,
-                                                        int N, int K, int kchunk) {
-  __shared__ __align__(16) __nv_bfloat16 As[TM][PADK];
-  __shared__ __align__(16) __nv_bfloat16 Bs[TN][PADK];
-  const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
-  const int kb = blockIdx.z * kchunk, ke = min(K, kb + kchunk);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
-  const int g = lane >> 2, tg = lane & 3;
-  float acc[2][4][4];
+constexpr int kRowsThreads = 512;
+__device__ __forceinline__ void pair_sync(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
+
+template <bool TRAIN>
+__global__ void __launch_bounds__(kRowsThreads) mlp_rows_kernel(const RowsArgs a) {
+  extern __shared__ __align__(16) __nv_bfloat16 wsm[];
+  __nv_bfloat16 *xsm = wsm + kWRows * kWPitch;  // two buffers of 128 rows, the operands between layers
+  __shared__ float sums[5 * HID + 2];  // db of the four layers, dw5, db5, loss
+  __shared__ float outs[2][128];       // the two halves of the output sums
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31, g = lane >> 2, tg = lane & 3;
+  const int pair = warp >> 1, c0 = (warp & 1) * (HID / 2);  // 16 rows, 64 columns
+  for (int q = t; q < kWRows * HID / 8; q += kRowsThreads)
+    cp16(wsm + (q / (HID / 8)) * kWPitch + (q % (HID / 8)) * 8, a.Wb + (long)q * 8);
+  if (TRAIN)
+    for (int q = t; q < 5 * HID + 2; q += kRowsThreads) sums[q] = 0.0f;
+  asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  const int r0 = blockIdx.x * 128 + pair * 16;
+  if (r0 < a.n) {
+    // this lane's row of an ldmatrix: matrix lane / 8, row lane % 8
+    const int mi = lane >> 3, ri = lane & 7;
+    uint32_t af[8][4];  // the layer's operand: 16 rows, all columns
+    const long ra = (long)(r0 + g), rb = ra + 8;
+    // the pair's rows of the operand buffers: where this lane writes and reads
+    __nv_bfloat16 *put = xsm + (pair * 16 + g) * kWPitch + 2 * tg + c0;
+    const __nv_bfloat16 *get = xsm + (pair * 16 + (mi & 1) * 8 + ri) * kWPitch + (mi >> 1) * 8;
+    constexpr int kBuf = 128 * kWPitch;
 #pragma unroll
-  for (int a = 0; a < 2; ++a)
-#pragma unroll
-    for (int b = 0; b < 4; ++b)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) acc[a][b][c] = 0.0f;
-  for (int k0 = kb; k0 < ke; k0 += TK) {
-    load_tile<!AT>(As, A, AT ? M : K, m0, M, k0);
-    load_tile<BT>(Bs, B, BT ? K : N, n0, N, k0);
-    __syncthreads();
-#pragma unroll
-    for (int ks = 0; ks < TK; ks += 16) {
-      uint32_t af[2][4], bf[4][2];
-#pragma unroll
-      for (int mt = 0; mt < 2; ++mt) {
-        const int r = wm + mt * 16 + g, c = ks + tg * 2;
-        af[mt][0] = *reinterpret_cast<const uint32_t *>(&As[r][c]);
-        af[mt][1] = *reinterpret_cast<const uint32_t *>(&As[r + 8][c]);
-        af[mt][2] = *reinterpret_cast<const uint32_t *>(&As[r][c + 8]);
-        af[mt][3] = *reinterpret_cast<const uint32_t *>(&As[r + 8][c + 8]);
-      }
-#pragma unroll
-      for (int nt = 0; nt < 4; ++nt) {
-        const int n = wn + nt * 8 + g, c = ks + tg * 2;
-        bf[nt][0] = *reinterpret_cast<const uint32_t *>(&Bs[n][c]);
-        bf[nt][1] = *reinterpret_cast<const uint32_t *>(&Bs[n][c + 8]);
-      }
-#pragma unroll
-      for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt) mma16816(acc[mt][nt], af[mt], bf[nt]);
+    for (int ks = 0; ks < IN / 16; ++ks) {
+      const __nv_bfloat16 *p = a.X + ra * IN + ks * 16 + 2 * tg, *q = a.X + rb * IN + ks * 16 + 2 * tg;
+      af[ks][0] = *(const uint32_t *)p;
+      af[ks][1] = *(const uint32_t *)q;
+      af[ks][2] = *(const uint32_t *)(p + 8);
+      af[ks][3] = *(const uint32_t *)(q + 8);
     }
-    __syncthreads();
-  }
+    float acc[8][4];
+    uint32_t last[8][2];  // the last layer's activations
 #pragma unroll
-  for (int mt = 0; mt < 2; ++mt)
+    for (int l = 0; l < 4; ++l) {
+      const int wr = l == 0 ? 0 : IN + (l - 1) * HID;  // first weight row of the layer
 #pragma unroll
-    for (int nt = 0; nt < 4; ++nt)
+      for (int nt = 0; nt < 8; ++nt)
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int r = m0 + wm + mt * 16 + g + 8 * h;
-        const int c = n0 + wn + nt * 8 + tg * 2;
-        if (r >= M) continue;
+        for (int e = 0; e < 4; ++e) acc[nt][e] = 0.0f;
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          if (c + e >= N) continue;
-          float *dst = C + (long)r * N + c + e;
-          if (ATOMIC) atomicAdd(dst, acc[mt][nt][2 * h + e]);
-          else *dst = acc[mt][nt][2 * h + e];
+      for (int ks = 0; ks < (l == 0 ? IN : HID) / 16; ++ks)
+#pragma unroll
+        for (int nt = 0; nt < 8; nt += 2) {
+          uint32_t bf[4];
+          ldsm4t(bf, wsm + (wr + ks * 16 + (mi & 1) * 8 + ri) * kWPitch + c0 + nt * 8 + (mi >> 1) * 8);
+          mma16816(acc[nt], af[ks], bf[0], bf[1]);
+          mma16816(acc[nt + 1], af[ks], bf[2], bf[3]);
+        }
+      const float *bias = a.P + off_b(l);
+#pragma unroll
+      for (int nt = 0; nt < 8; ++nt) {
+        const int c = c0 + nt * 8 + 2 * tg;
+        const float2 bc = *(const float2 *)(bias + c);
+        float y[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float z = acc[nt][e] + (e & 1 ? bc.y : bc.x), s = sigm(z);
+          y[e] = z * s;
+          if (TRAIN) acc[nt][e] = s * (1.0f + z * (1.0f - s));
+        }
+        const uint32_t ya = pack2(y[0], y[1]), yb = pack2(y[2], y[3]);
+        if (l < 3) {
+          *(uint32_t *)(put + (l & 1) * kBuf + nt * 8) = ya;
+          *(uint32_t *)(put + (l & 1) * kBuf + 8 * kWPitch + nt * 8) = yb;
+        }
+        last[nt][0] = ya;
+        last[nt][1] = yb;
+        if (TRAIN && l < 3) {
+          *(uint32_t *)(a.A[l] + ra * HID + c) = ya;
+          *(uint32_t *)(a.A[l] + rb * HID + c) = yb;
+          *(float2 *)(a.Z[l] + ra * HID + c) = make_float2(acc[nt][0], acc[nt][1]);
+          *(float2 *)(a.Z[l] + rb * HID + c) = make_float2(acc[nt][2], acc[nt][3]);
         }
       }
-}
-
-// ---- elementwise pieces ---------------------------------------------------------
-__device__ __forceinline__ float sigm(float z) { return 1.0f / (1.0f + expf(-z)); }
-
-__global__ void bias_silu_kernel(float *Z, const float *__restrict__ b, __nv_bfloat16 *Aout, long n) {
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float z = Z[i] + b[i % HID];
-  Z[i] = z;
-  Aout[i] = __float2bfloat16_rn(z * sigm(z));
-}
-
-// one block of HID threads walks rows [r0, r1); thread k owns hidden unit k.
-// Without targets (y == nullptr) only out is written.
-__global__ void __launch_bounds__(HID) out_layer_kernel(const __nv_bfloat16 *__restrict__ A4,
-                                                         const float *__restrict__ Z4,
-                                                         const float *__restrict__ P, float *out,
-                                                         const float *__restrict__ y, int n, int rows_per_block,
-                                                         float *grad, __nv_bfloat16 *dZ4, float *loss) {
-  __shared__ float red[HID / 32];
-  __shared__ float rowsum;
-  const int k = threadIdx.x;
-  const float w5 = P[kOffW5 + k], b5 = P[kOffW5 + HID];
-  float gw = 0.0f, gb = 0.0f, ls = 0.0f;
-  const int r0 = blockIdx.x * rows_per_block, r1 = min(n, r0 + rows_per_block);
-  for (int r = r0; r < r1; ++r) {
-    const float a = __bfloat162float(A4[(long)r * HID + k]);
-    float v = a * w5;
+      if (l < 3) {
+        pair_sync(1 + pair);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if ((k & 31) == 0) red[k >> 5] = v;
-    __syncthreads();
-    if (k == 0) {
-      float s = b5;
-      for (int q = 0; q < HID / 32; ++q) s += red[q];
-      rowsum = s;
-      out[r] = s;
-    }
-    __syncthreads();
-    if (y) {
-      const float o = rowsum;
-      const float d = 2.0f * (o - y[r]) / (float)n;
-      if (k == 0) {
-        ls += (o - y[r]) * (o - y[r]);
-        gb += d;
+        for (int ks = 0; ks < HID / 16; ++ks) ldsm4(af[ks], get + (l & 1) * kBuf + ks * 16);
       }
-      gw += d * a;
-      const float z = Z4[(long)r * HID + k];
-      const float s = sigm(z);
-      dZ4[(long)r * HID + k] = __float2bfloat16_rn(d * w5 * (s * (1.0f + z * (1.0f - s))));
+    }
+    // out = A4 w5 + b5
+    const float *w5 = a.P + kOffW5;
+    float oa = 0.0f, ob = 0.0f;
+#pragma unroll
+    for (int nt = 0; nt < 8; ++nt) {
+      const float2 w = *(const float2 *)(w5 + c0 + nt * 8 + 2 * tg);
+      const float2 u = unpack2(last[nt][0]), v = unpack2(last[nt][1]);
+      oa = fmaf(u.x, w.x, fmaf(u.y, w.y, oa));
+      ob = fmaf(v.x, w.x, fmaf(v.y, w.y, ob));
+    }
+#pragma unroll
+    for (int o = 1; o < 4; o <<= 1) {
+      oa += __shfl_xor_sync(0xffffffffu, oa, o);
+      ob += __shfl_xor_sync(0xffffffffu, ob, o);
+    }
+    if (tg == 0) {
+      outs[warp & 1][pair * 16 + g] = oa;
+      outs[warp & 1][pair * 16 + g + 8] = ob;
+    }
+    pair_sync(1 + pair);
+    oa = outs[0][pair * 16 + g] + outs[1][pair * 16 + g] + w5[HID];
+    ob = outs[0][pair * 16 + g + 8] + outs[1][pair * 16 + g + 8] + w5[HID];
+    if (tg == 0 && c0 == 0) {
+      a.out[ra] = oa;
+      a.out[rb] = ob;
+    }
+    if (TRAIN) {
+      const float ea = oa - a.y[ra], eb = ob - a.y[rb];
+      const float da = 2.0f * ea / (float)a.n, db = 2.0f * eb / (float)a.n;
+      if (tg == 0 && c0 == 0) {
+        atomicAdd(sums + 5 * HID, da + db);
+        atomicAdd(sums + 5 * HID + 1, ea * ea + eb * eb);
+      }
+#pragma unroll
+      for (int l = 3; l >= 0; --l) {
+        // acc: silu' of layer 3, or dA of layer l; dZ_l out and into the next operand
+#pragma unroll
+        for (int nt = 0; nt < 8; ++nt) {
+          const int c = c0 + nt * 8 + 2 * tg;
+          uint32_t fa, fb;
+          if (l == 3) {
+            const float2 u = unpack2(last[nt][0]), v = unpack2(last[nt][1]), w = *(const float2 *)(w5 + c);
+            add_columns(sums + 4 * HID + c0 + nt * 8, da * u.x + db * v.x, da * u.y + db * v.y, lane);
+            fa = pack2(da * w.x * acc[nt][0], da * w.y * acc[nt][1]);
+            fb = pack2(db * w.x * acc[nt][2], db * w.y * acc[nt][3]);
+          } else {
+            const float2 u = *(const float2 *)(a.Z[l] + ra * HID + c), v = *(const float2 *)(a.Z[l] + rb * HID + c);
+            fa = pack2(acc[nt][0] * u.x, acc[nt][1] * u.y);
+            fb = pack2(acc[nt][2] * v.x, acc[nt][3] * v.y);
+          }
+          if (l > 0) {
+            *(uint32_t *)(put + (l & 1) * kBuf + nt * 8) = fa;
+            *(uint32_t *)(put + (l & 1) * kBuf + 8 * kWPitch + nt * 8) = fb;
+          }
+          *(uint32_t *)(a.dZ[l] + ra * HID + c) = fa;
+          *(uint32_t *)(a.dZ[l] + rb * HID + c) = fb;
+          const float2 u = unpack2(fa), v = unpack2(fb);
+          add_columns(sums + l * HID + c0 + nt * 8, u.x + v.x, u.y + v.y, lane);
+        }
+        if (l == 0) break;
+        pair_sync(1 + pair);
+#pragma unroll
+        for (int ks = 0; ks < HID / 16; ++ks) ldsm4(af[ks], get + (l & 1) * kBuf + ks * 16);
+        const int wr = IN + (l - 1) * HID;
+#pragma unroll
+        for (int nt = 0; nt < 8; ++nt)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc[nt][e] = 0.0f;
+#pragma unroll
+        for (int ks = 0; ks < HID / 16; ++ks)
+#pragma unroll
+          for (int nt = 0; nt < 8; nt += 2) {
+            uint32_t bf[4];  // columns of W_l^T: rows of W_l
+            ldsm4(bf, wsm + (wr + c0 + nt * 8 + (mi >> 1) * 8 + ri) * kWPitch + ks * 16 + (mi & 1) * 8);
+            mma16816(acc[nt], af[ks], bf[0], bf[1]);
+            mma16816(acc[nt + 1], af[ks], bf[2], bf[3]);
+          }
+      }
     }
   }
-  if (y) {
-    atomicAdd(grad + kOffW5 + k, gw);
-    if (k == 0) {
-      atomicAdd(grad + kOffW5 + HID, gb);
-      atomicAdd(loss, ls / (float)n);
+  if (TRAIN) {
+    __syncthreads();
+    for (int q = t; q < 5 * HID; q += kRowsThreads)
+      atomicAdd(a.grad + (q < 4 * HID ? off_b(q / HID) + q % HID : kOffW5 + q % HID), sums[q]);
+    if (t == 0) {
+      atomicAdd(a.grad + kOffW5 + HID, sums[5 * HID]);
+      atomicAdd(a.loss, sums[5 * HID + 1] / (float)a.n);
     }
   }
 }
 
-__global__ void silu_back_kernel(const float *__restrict__ dA, const float *__restrict__ Z, __nv_bfloat16 *dZ,
-                                 long n) {
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float z = Z[i];
-  const float s = sigm(z);
-  dZ[i] = __float2bfloat16_rn(dA[i] * (s * (1.0f + z * (1.0f - s))));
-}
+// ---- weight gradients ---------------------------------------------------------------
+// dW_l += A_{l-1}^T dZ_l of rows [z chunk, (z + 1) chunk) for layer blockIdx.x:
+// the whole fan_in x 128 product in one block's registers (16 rows of dW per
+// warp), 64 rows of both operands at a time through shared memory, fetched
+// ahead by cp.async; the partial sums of the row chunks meet in FP32 atomics.
+constexpr int kGradRows = 64;
+constexpr int kGradSmem = 2 * 2 * kGradRows * kWPitch * 2;
 
-// db[c] += sum over rows of dZ[r][c]; block = HID threads, 256 rows each
-__global__ void colsum_kernel(const __nv_bfloat16 *__restrict__ dZ, int n, float *db) {
-  const int c = threadIdx.x;
-  const int r0 = blockIdx.x * 256, r1 = min(n, r0 + 256);
-  float s = 0.0f;
-  for (int r = r0; r < r1; ++r) s += __bfloat162float(dZ[(long)r * HID + c]);
-  atomicAdd(db + c, s);
+__global__ void __launch_bounds__(256) mlp_weight_grad_kernel(const RowsArgs a, int chunk) {
+  extern __shared__ __align__(16) __nv_bfloat16 gsm[];
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31, g = lane >> 2, tg = lane & 3;
+  const int l = blockIdx.x, fi = l == 0 ? IN : HID;
+  const __nv_bfloat16 *A = l == 0 ? a.X : a.A[l - 1], *D = a.dZ[l];
+  const int r0 = blockIdx.y * chunk, r1 = min(a.n, r0 + chunk);
+  auto fetch = [&](int buf, int r) {  // rows r .. r + 63 (a multiple of 64 rows in all)
+    __nv_bfloat16 *sa = gsm + buf * 2 * kGradRows * kWPitch, *sd = sa + kGradRows * kWPitch;
+    for (int q = t; q < kGradRows * fi / 8; q += 256) cp16(sa + (q / (fi / 8)) * kWPitch + (q % (fi / 8)) * 8, A + (long)r * fi + (long)q * 8);
+    for (int q = t; q < kGradRows * HID / 8; q += 256) cp16(sd + (q / (HID / 8)) * kWPitch + (q % (HID / 8)) * 8, D + (long)r * HID + (long)q * 8);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  float acc[16][4];
+#pragma unroll
+  for (int nt = 0; nt < 16; ++nt)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[nt][e] = 0.0f;
+  const int mi = lane >> 3, ri = lane & 7;
+  if (r0 < r1) fetch(0, r0);
+  int buf = 0;
+  for (int r = r0; r < r1; r += kGradRows, buf ^= 1) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    if (r + kGradRows < r1) fetch(buf ^ 1, r + kGradRows);
+    const __nv_bfloat16 *sa = gsm + buf * 2 * kGradRows * kWPitch, *sd = sa + kGradRows * kWPitch;
+    if (warp * 16 < fi) {
+#pragma unroll
+      for (int ks = 0; ks < kGradRows / 16; ++ks) {
+        uint32_t af[4];
+        ldsm4t(af, sa + (ks * 16 + (mi >> 1) * 8 + ri) * kWPitch + warp * 16 + (mi & 1) * 8);
+#pragma unroll
+        for (int nt = 0; nt < 16; nt += 2) {
+          uint32_t bf[4];
+          ldsm4t(bf, sd + (ks * 16 + (mi & 1) * 8 + ri) * kWPitch + nt * 8 + (mi >> 1) * 8);
+          mma16816(acc[nt], af, bf[0], bf[1]);
+          mma16816(acc[nt + 1], af, bf[2], bf[3]);
+        }
+      }
+    }
+    __syncthreads();
+  }
+  if (warp * 16 >= fi || r0 >= r1) return;
+  float *G = a.grad + off_w(l) + (long)(warp * 16 + g) * HID + 2 * tg;
+#pragma unroll
+  for (int nt = 0; nt < 16; ++nt)
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(G + h * 8 * HID + nt * 8), "f"(acc[nt][2 * h]),
+                   "f"(acc[nt][2 * h + 1])
+                   : "memory");
 }
 
 struct AdamArgs {
   float lr, b1, b2, eps, c1, c2;  // c1 = 1/(1-b1^t), c2 = 1/(1-b2^t)
 };
 
-__global__ void adam_kernel(float *P, const float *__restrict__ G, float *Mo, float *Vo, AdamArgs a, int n) {
+// the BF16 copy of weight i of the flat layout, -1 for biases and w5
+__device__ __forceinline__ int wb_index(int i) {
+#pragma unroll
+  for (int l = 0; l < 4; ++l)
+    if (i >= off_w(l) && i < off_b(l)) return (l == 0 ? 0 : IN * HID + (l - 1) * HID * HID) + i - off_w(l);
+  return -1;
+}
+
+// Adam step and the refreshed BF16 copy
+__global__ void adam_kernel(float *P, const float *__restrict__ G, float *Mo, float *Vo, __nv_bfloat16 *Wb, AdamArgs a,
+                            int n) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float g = G[i];
@@ -285,7 +405,10 @@ __global__ void adam_kernel(float *P, const float *__restrict__ G, float *Mo, fl
   const float v = a.b2 * Vo[i] + (1.0f - a.b2) * g * g;
   Mo[i] = m;
   Vo[i] = v;
-  P[i] -= a.lr * (m * a.c1) / (sqrtf(v * a.c2) + a.eps);
+  const float p = P[i] - a.lr * (m * a.c1) / (sqrtf(v * a.c2) + a.eps);
+  P[i] = p;
+  const int w = wb_index(i);
+  if (w >= 0) Wb[w] = __float2bfloat16_rn(p);
 }
 
 // BF16 copies of W1..W4 in the [K][N] layout of the forward products
@@ -714,7 +837,6 @@ __global__ void __launch_bounds__(tc::kThreads, 1) mlp_forward_tc_kernel(const d
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256u) : "memory");
 }
 
-long wb_off(int l) { return l == 0 ? 0 : (long)IN * HID + (long)(l - 1) * HID * HID; }
 
 }  // namespace
 
@@ -724,11 +846,10 @@ struct nrgpu_mlp {
   float *P, *G, *Mo, *Vo;  // master params, gradients, Adam moments
   __nv_bfloat16 *Wb;       // BF16 W1..W4
   __nv_bfloat16 *X;        // [max_batch][IN]
-  float *Z[4];             // [max_batch][HID] pre-activations
-  __nv_bfloat16 *Ab[4];    // [max_batch][HID] activations
-  float *dA;               // [max_batch][HID]
-  __nv_bfloat16 *dZ;       // [max_batch][HID]
-  float *out, *y, *loss;
+  float *Z[4];             // [max_batch][HID] silu' of the pre-activations (1 to 3)
+  __nv_bfloat16 *Ab[4];    // [max_batch][HID] activations (1 to 3)
+  __nv_bfloat16 *dZ[4];    // [max_batch][HID] pre-activation gradients
+  float *out, *loss;       // loss: right after G
   double *cond;            // the conditioning table
   int ncond;
   int *d_tcstatus;         // a wait of the tensor-core forward ran out
@@ -737,41 +858,22 @@ struct nrgpu_mlp {
 
 namespace {
 
-int check_dims(int M, int N, int K) {
-  if (M % 16 || N % 16 || K % TK || M <= 0 || N <= 0 || K <= 0)
-    return nrgpu_set_error(NRGPU_ERR_ARG, "gemm dims %d x %d x %d (M, N multiples of 16, K of 32)", M, N, K);
-  return NRGPU_OK;
-}
-
-template <bool AT, bool BT>
-int gemm(const __nv_bfloat16 *A, const __nv_bfloat16 *B, float *C, int M, int N, int K, int splits,
-         cudaStream_t st) {
-  int e = check_dims(M, N, K);
-  if (e) return e;
-  const dim3 grid((N + TN - 1) / TN, (M + TM - 1) / TM, 1);
-  if (splits > 1) {
-    int kc = (K + splits - 1) / splits;
-    kc = (kc + TK - 1) / TK * TK;
-    NRGPU_CUDA_TRY(cudaMemsetAsync(C, 0, sizeof(float) * (size_t)M * N, st));
-    gemm_bf16_kernel<AT, BT, true><<<dim3(grid.x, grid.y, (K + kc - 1) / kc), 128, 0, st>>>(A, B, C, M, N, K, kc);
-  } else {
-    gemm_bf16_kernel<AT, BT, false><<<grid, 128, 0, st>>>(A, B, C, M, N, K, K);
-  }
-  NRGPU_CUDA_TRY(cudaGetLastError());
-  return NRGPU_OK;
-}
-
 inline int nb(long n, int t = 256) { return (int)((n + t - 1) / t); }
 
-// forward of n rows already featurised in M->X; fills Z, Ab
-int forward(nrgpu_mlp *M, int n, cudaStream_t st) {
-  const __nv_bfloat16 *in = M->X;
+RowsArgs rows_args(nrgpu_mlp *M, int n, const float *y, float *out) {
+  RowsArgs a = {M->X, M->Wb, M->P, y, out, {}, {}, {}, M->G, M->loss, n};
   for (int l = 0; l < 4; ++l) {
-    int e = gemm<false, false>(in, M->Wb + wb_off(l), M->Z[l], n, HID, fan_in(l), 1, st);
-    if (e) return e;
-    bias_silu_kernel<<<nb((long)n * HID), 256, 0, st>>>(M->Z[l], M->P + off_b(l), M->Ab[l], (long)n * HID);
-    in = M->Ab[l];
+    a.Z[l] = M->Z[l];
+    a.A[l] = M->Ab[l];
+    a.dZ[l] = M->dZ[l];
   }
+  return a;
+}
+
+// network output of n rows already featurised in M->X
+int forward(nrgpu_mlp *M, int n, float *out, cudaStream_t st) {
+  NRGPU_CUDA_TRY(cudaFuncSetAttribute(mlp_rows_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowsSmem));
+  mlp_rows_kernel<false><<<nb(n, 128), kRowsThreads, kRowsSmem, st>>>(rows_args(M, n, nullptr, out));
   NRGPU_CUDA_TRY(cudaGetLastError());
   return NRGPU_OK;
 }
@@ -803,24 +905,22 @@ extern "C" int nrgpu_mlp_create(int max_batch, nrgpu_mlp **out) {
   M->max_batch = max_batch;
   const size_t nh = (size_t)max_batch * HID;
   bool ok = cudaMalloc(&M->P, sizeof(float) * kNParams) == cudaSuccess &&
-            cudaMalloc(&M->G, sizeof(float) * kNParams) == cudaSuccess &&
+            cudaMalloc(&M->G, sizeof(float) * (kNParams + 1)) == cudaSuccess &&
             cudaMalloc(&M->Mo, sizeof(float) * kNParams) == cudaSuccess &&
             cudaMalloc(&M->Vo, sizeof(float) * kNParams) == cudaSuccess &&
             cudaMalloc(&M->Wb, sizeof(__nv_bfloat16) * (IN * HID + 3 * HID * HID)) == cudaSuccess &&
             cudaMalloc(&M->X, sizeof(__nv_bfloat16) * (size_t)max_batch * IN) == cudaSuccess &&
-            cudaMalloc(&M->dA, sizeof(float) * nh) == cudaSuccess &&
-            cudaMalloc(&M->dZ, sizeof(__nv_bfloat16) * nh) == cudaSuccess &&
             cudaMalloc(&M->out, sizeof(float) * max_batch) == cudaSuccess &&
-            cudaMalloc(&M->y, sizeof(float) * max_batch) == cudaSuccess &&
-            cudaMalloc(&M->loss, sizeof(float)) == cudaSuccess &&
             cudaMalloc(&M->d_tcstatus, sizeof(int)) == cudaSuccess &&
             cudaMemset(M->d_tcstatus, 0, sizeof(int)) == cudaSuccess;
   for (int l = 0; l < 4 && ok; ++l)
-    ok = cudaMalloc(&M->Z[l], sizeof(float) * nh) == cudaSuccess &&
-         cudaMalloc(&M->Ab[l], sizeof(__nv_bfloat16) * nh) == cudaSuccess;
+    ok = (l == 3 || cudaMalloc(&M->Z[l], sizeof(float) * nh) == cudaSuccess) &&
+         (l == 3 || cudaMalloc(&M->Ab[l], sizeof(__nv_bfloat16) * nh) == cudaSuccess) &&
+         cudaMalloc(&M->dZ[l], sizeof(__nv_bfloat16) * nh) == cudaSuccess;
+  M->loss = M->G + kNParams;
   if (ok)
     ok = cudaMemset(M->P, 0, sizeof(float) * kNParams) == cudaSuccess &&
-         cudaMemset(M->G, 0, sizeof(float) * kNParams) == cudaSuccess &&
+         cudaMemset(M->G, 0, sizeof(float) * (kNParams + 1)) == cudaSuccess &&
          cudaMemset(M->Mo, 0, sizeof(float) * kNParams) == cudaSuccess &&
          cudaMemset(M->Vo, 0, sizeof(float) * kNParams) == cudaSuccess;
   if (!ok) {
@@ -835,11 +935,12 @@ extern "C" int nrgpu_mlp_create(int max_batch, nrgpu_mlp **out) {
 extern "C" int nrgpu_mlp_destroy(nrgpu_mlp *M) {
   if (!M) return NRGPU_OK;
   cudaFree(M->P); cudaFree(M->G); cudaFree(M->Mo); cudaFree(M->Vo); cudaFree(M->Wb); cudaFree(M->X);
-  cudaFree(M->dA); cudaFree(M->dZ); cudaFree(M->out); cudaFree(M->y); cudaFree(M->loss); cudaFree(M->cond);
+  cudaFree(M->out); cudaFree(M->cond);
   cudaFree(M->d_tcstatus);
   for (int l = 0; l < 4; ++l) {
     cudaFree(M->Z[l]);
     cudaFree(M->Ab[l]);
+    cudaFree(M->dZ[l]);
   }
   free(M);
   return NRGPU_OK;
@@ -890,38 +991,23 @@ extern "C" int nrgpu_mlp_train_step(nrgpu_mlp *M, const float *d_y, int n, float
   if (!M || !d_y || n < 64 || n % 64 || n > M->max_batch)
     return nrgpu_set_error(NRGPU_ERR_ARG, "batch %d: a multiple of 64 up to %d", n, M ? M->max_batch : 0);
   const cudaStream_t st = (cudaStream_t)stream;
-  int e = forward(M, n, st);
-  if (e) return e;
-  NRGPU_CUDA_TRY(cudaMemsetAsync(M->G, 0, sizeof(float) * kNParams, st));
-  NRGPU_CUDA_TRY(cudaMemsetAsync(M->loss, 0, sizeof(float), st));
-  const int rpb = 64;
-  out_layer_kernel<<<(n + rpb - 1) / rpb, HID, 0, st>>>(M->Ab[3], M->Z[3], M->P, M->out, d_y, n, rpb, M->G, M->dZ,
-                                                        M->loss);
+  NRGPU_CUDA_TRY(cudaMemsetAsync(M->G, 0, sizeof(float) * (kNParams + 1), st));  // the gradients and the loss
+  NRGPU_CUDA_TRY(cudaFuncSetAttribute(mlp_rows_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowsSmem));
+  NRGPU_CUDA_TRY(cudaFuncSetAttribute(mlp_weight_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGradSmem));
+  const RowsArgs a = rows_args(M, n, d_y, M->out);
+  mlp_rows_kernel<true><<<nb(n, 128), kRowsThreads, kRowsSmem, st>>>(a);
+  // row chunks: enough blocks (four layers each) for the SMs, at least 128
+  // rows each so that the atomics of a block's 128 x 128 sums stay few
+  const int chunk = max(128, (n + 36 * kGradRows - 1) / (36 * kGradRows) * kGradRows);
+  mlp_weight_grad_kernel<<<dim3(4, nb(n, chunk)), 256, kGradSmem, st>>>(a, chunk);
   NRGPU_CUDA_TRY(cudaGetLastError());
-  const int splits = max(1, min(64, n / 1024));
-  for (int l = 3; l >= 0; --l) {
-    // dW_l = A_{l-1}^T dZ_l straight into its [fan_in][HID] slot of G,
-    // db_l = column sums of dZ_l
-    const __nv_bfloat16 *Ain = l ? M->Ab[l - 1] : M->X;
-    e = gemm<true, false>(Ain, M->dZ, M->G + off_w(l), fan_in(l), HID, n, splits, st);
-    if (e) return e;
-    colsum_kernel<<<(n + 255) / 256, HID, 0, st>>>(M->dZ, n, M->G + off_b(l));
-    NRGPU_CUDA_TRY(cudaGetLastError());
-    if (l == 0) break;
-    // dA_{l-1} = dZ_l W_l^T, dZ_{l-1} = dA * silu'(Z_{l-1})
-    e = gemm<false, true>(M->dZ, M->Wb + wb_off(l), M->dA, n, HID, HID, 1, st);
-    if (e) return e;
-    silu_back_kernel<<<nb((long)n * HID), 256, 0, st>>>(M->dA, M->Z[l - 1], M->dZ, (long)n * HID);
-    NRGPU_CUDA_TRY(cudaGetLastError());
-  }
   if (update) {
     M->adam_t++;
-    AdamArgs a;
-    a.lr = lr; a.b1 = 0.9f; a.b2 = 0.999f; a.eps = 1e-8f;
-    a.c1 = (float)(1.0 / (1.0 - pow(0.9, (double)M->adam_t)));
-    a.c2 = (float)(1.0 / (1.0 - pow(0.999, (double)M->adam_t)));
-    adam_kernel<<<nb(kNParams), 256, 0, st>>>(M->P, M->G, M->Mo, M->Vo, a, kNParams);
-    refresh_bf16_kernel<<<nb(IN * HID + 3 * HID * HID), 256, 0, st>>>(M->P, M->Wb);
+    AdamArgs q;
+    q.lr = lr; q.b1 = 0.9f; q.b2 = 0.999f; q.eps = 1e-8f;
+    q.c1 = (float)(1.0 / (1.0 - pow(0.9, (double)M->adam_t)));
+    q.c2 = (float)(1.0 / (1.0 - pow(0.999, (double)M->adam_t)));
+    adam_kernel<<<nb(kNParams), 256, 0, st>>>(M->P, M->G, M->Mo, M->Vo, M->Wb, q, kNParams);
     NRGPU_CUDA_TRY(cudaGetLastError());
   }
   if (loss) {
@@ -941,13 +1027,7 @@ extern "C" int nrgpu_mlp_gradients(nrgpu_mlp *M, float *host_grad, int n_params)
 extern "C" int nrgpu_mlp_forward(nrgpu_mlp *M, int n, float *d_out, void *stream) {
   if (!M || !d_out || n < 16 || n % 16 || n > M->max_batch)
     return nrgpu_set_error(NRGPU_ERR_ARG, "rows %d: a multiple of 16 up to %d", n, M ? M->max_batch : 0);
-  const cudaStream_t st = (cudaStream_t)stream;
-  int e = forward(M, n, st);
-  if (e) return e;
-  out_layer_kernel<<<(n + 63) / 64, HID, 0, st>>>(M->Ab[3], M->Z[3], M->P, d_out, nullptr, n, 64, nullptr, nullptr,
-                                                  nullptr);
-  NRGPU_CUDA_TRY(cudaGetLastError());
-  return NRGPU_OK;
+  return forward(M, n, d_out, (cudaStream_t)stream);
 }
 
 extern "C" int nrgpu_mlp_predict_u(nrgpu_mlp *M, const double *host_cond, int m, double dx, double uscale, double *u,
@@ -963,10 +1043,7 @@ extern "C" int nrgpu_mlp_predict_u(nrgpu_mlp *M, const double *host_cond, int m,
     const int n16 = (n + 15) / 16 * 16;  // rows past np are computed and dropped
     mlp_features_kernel<<<nb(n16), 256, 0, st>>>(M->cond, nullptr, nullptr, first, n16, Feat{m, dx}, M->X);
     NRGPU_CUDA_TRY(cudaGetLastError());
-    e = forward(M, n16, st);
-    if (e) return e;
-    out_layer_kernel<<<(n16 + 63) / 64, HID, 0, st>>>(M->Ab[3], M->Z[3], M->P, M->out, nullptr, n16, 64, nullptr,
-                                                      nullptr, nullptr);
+    if ((e = forward(M, n16, M->out, st))) return e;
     scale_to_u_kernel<<<nb(n), 256, 0, st>>>(M->out, uscale, u + first, n);
     NRGPU_CUDA_TRY(cudaGetLastError());
   }
