@@ -17,107 +17,10 @@
 #include <cstdio>
 #include <cstring>
 #include <mutex>
-#include "nrgpu_level.cuh"
-#include "nrgpu_fd.cuh"
+#include "nrgpu_rhs.cuh"
 #include "nrgpu_tma.cuh"
 
 namespace {
-
-enum { G11 = 0, CHI = 6, A11 = 7, KK = 13, GA1 = 14, ALPHA = 17, BETA1 = 18, BB1 = 21 };
-
-// lopsided advection rows (numerators), row r = stencil shifted by r
-// (bam_amr_advection.h:28-66); denominators 2, 12, 60
-__constant__ double kAdv2[3][3] = {{3, -4, 1}, {1, 0, -1}, {-1, 4, -3}};
-__constant__ double kAdv4[5][5] = {{25, -48, 36, -16, 3}, {3, 10, -18, 6, -1}, {-1, 8, 0, -8, 1},
-                                   {1, -6, 18, -10, -3}, {-3, 16, -36, 48, -25}};
-__constant__ double kAdv6[7][7] = {{147, -360, 450, -400, 225, -72, 10}, {10, 77, -150, 100, -50, 15, -2},
-                                   {-2, 24, 35, -80, 30, -8, 1},        {1, -9, 45, 0, -45, 9, -1},
-                                   {-1, 8, -30, 80, -35, -24, 2},       {2, -15, 50, -100, 150, -77, -10},
-                                   {-10, 72, -225, 400, -450, 360, -147}};
-
-struct AdvDir {
-  int base;     // offset of tap 0 relative to the point
-  int step;     // +-stride between taps (0 when the shift is zero)
-  int row;      // stencil row
-};
-
-// direction setup of set_advectionN_onedir (bam_amr_advection.h:72-192)
-__device__ __forceinline__ AdvDir adv_dir(int i, int imax, double w, int q, int lop, int s) {
-  AdvDir a;
-  int rst = q - lop, offset, wsign;
-  if (w < 0) { wsign = -1; offset = (i >= rst) ? 0 : rst - i; }
-  else if (w > 0) { wsign = 1; offset = (imax - i >= rst) ? 0 : rst - (imax - i); }
-  else { wsign = 0; offset = 0; }
-  offset += lop;
-  a.row = offset;
-  a.step = wsign * s;
-  a.base = -offset * wsign * s;
-  return a;
-}
-
-template <int Q>
-__device__ __forceinline__ double adv_sum(const double *__restrict__ f, int x, const AdvDir ad[3],
-                                          const double cw[3]) {
-  double acc = 0.0;
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    double t = 0.0;
-    const int p0 = x + ad[d].base;
-#pragma unroll
-    for (int n = 0; n <= Q; ++n) {
-      const double c = Q == 2 ? kAdv2[ad[d].row][n] : Q == 4 ? kAdv4[ad[d].row][n] : kAdv6[ad[d].row][n];
-      t += c * ldg(f + p0 + n * ad[d].step);
-    }
-    acc += cw[d] * t;
-  }
-  return acc;
-}
-
-// Kreiss-Oliger: sum over directions of undivided differences / h
-template <int OD>
-__device__ __forceinline__ double ko_sum(const double *__restrict__ f, int x, const int st[3],
-                                         const double ooh[3]) {
-  double acc = 0.0;
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    const int s = st[d];
-    double t;
-    if (OD == 4)
-      t = 6.0 * ldg(f + x) - 4.0 * (ldg(f + x - s) + ldg(f + x + s)) + (ldg(f + x - 2 * s) + ldg(f + x + 2 * s));
-    else
-      t = (ldg(f + x - 3 * s) + ldg(f + x + 3 * s)) - 6.0 * (ldg(f + x - 2 * s) + ldg(f + x + 2 * s)) +
-          15.0 * (ldg(f + x - s) + ldg(f + x + s)) - 20.0 * ldg(f + x);
-    acc += ooh[d] * t;
-  }
-  return OD == 4 ? -acc : acc;
-}
-
-// Kreiss-Oliger with FP32 sums of centre-relative taps (the weights sum to
-// zero); P = 0 keeps FP64
-template <int OD, int P>
-__device__ __forceinline__ double ko_p(const double *__restrict__ f, int x, const int st[3], const double ooh[3]) {
-  if (P == 0) return ko_sum<OD>(f, x, st, ooh);
-  const double c = ldg(f + x);
-  double acc = 0.0;
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    const int s = st[d];
-    float t;
-    if (OD == 4)
-      t = -4.0f * (tapf(f, x, -1, s, c) + tapf(f, x, 1, s, c)) + (tapf(f, x, -2, s, c) + tapf(f, x, 2, s, c));
-    else
-      t = (tapf(f, x, -3, s, c) + tapf(f, x, 3, s, c)) - 6.0f * (tapf(f, x, -2, s, c) + tapf(f, x, 2, s, c)) +
-          15.0f * (tapf(f, x, -1, s, c) + tapf(f, x, 1, s, c));
-    acc += ooh[d] * (double)t;
-  }
-  return OD == 4 ? -acc : acc;
-}
-
-struct PointCtx {
-  int ijk, i, j, k, imax, jmax, kmax, dist;
-  int st[3];
-  double h[3];
-};
 
 // ---- the per-point right-hand side -------------------------------------------
 template <int ORD, int CSY = 0, int CSZ = 0>
@@ -491,47 +394,6 @@ __device__ __forceinline__ void bssn_point(const CVarPtrs &U, const PointCtx &P,
 }
 
 // ---- epilogues ----------------------------------------------------------------
-// a hint that the line holding p will be read soon: fetched into L2, no
-// register written (PTX prefetch.global.L2)
-__device__ __forceinline__ void l2_prefetch(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
-
-enum { EPI_RHS = 0, EPI_ADDLINEAR = 1, EPI_RK = 2 };
-
-// EPI_RK accumulator modes: ACC_ADD acc += wacc rhs; ACC_INIT acc = upre +
-// wacc rhs (the first stage, so that the step needs no copy of u); ACC_FINAL
-// out = acc + wacc rhs (the last stage writes u from the accumulator)
-enum { ACC_ADD = 0, ACC_INIT = 1, ACC_FINAL = 2 };
-
-struct Epilogue {
-  int mode;
-  double c;        // EPI_ADDLINEAR: unew = upre + c rhs
-  double wacc;     // EPI_RK: acc += wacc * rhs
-  double cv;       // EPI_RK: vout = upre + cv * rhs (when has_v)
-  int has_v;
-  int accmode;     // EPI_RK: ACC_ADD / ACC_INIT / ACC_FINAL
-};
-
-__device__ __forceinline__ void det_trace_fix(double n[NRGPU_NV], const nrgpu_bssn_params &p) {
-  double *g = n + G11, *A = n + A11;
-  const double detg = g[0] * g[3] * g[5] + 2.0 * g[1] * g[2] * g[4] - g[0] * g[4] * g[4] -
-                      g[3] * g[2] * g[2] - g[5] * g[1] * g[1];
-  const double detnginv = 1.0 / detg;
-  if (p.subtractA) {
-    const double gi0 = g[3] * g[5] - g[4] * g[4], gi1 = g[2] * g[4] - g[1] * g[5],
-                 gi2 = g[1] * g[4] - g[2] * g[3], gi3 = g[0] * g[5] - g[2] * g[2],
-                 gi4 = g[1] * g[2] - g[0] * g[4], gi5 = g[0] * g[3] - g[1] * g[1];
-    const double trA = detnginv * (gi0 * A[0] + gi3 * A[3] + gi5 * A[5] + 2.0 * (gi1 * A[1] + gi2 * A[2] + gi4 * A[4]));
-    const double aux = -trA / 3.0;
-#pragma unroll
-    for (int v = 0; v < 6; ++v) A[v] += aux * g[v];
-  }
-  if (p.normalizedetg) {
-    const double aux = cbrt(detnginv);
-#pragma unroll
-    for (int v = 0; v < 6; ++v) g[v] *= aux;
-  }
-}
-
 __device__ __forceinline__ void store(const double r[NRGPU_NV], int x, const VarPtrs &out, const CVarPtrs &pre,
                                       const VarPtrs &acc, const Epilogue &E, const nrgpu_bssn_params &p) {
   if (E.mode == EPI_RHS) {
@@ -542,7 +404,7 @@ __device__ __forceinline__ void store(const double r[NRGPU_NV], int x, const Var
 #pragma unroll
     for (int v = 0; v < NRGPU_NV; ++v) n[v] = ldg(pre.p[v] + x) + E.c * r[v];
     n[KK] = p.forceKzerofactor * n[KK];
-    det_trace_fix(n, p);
+    det_trace_fix(n, p.subtractA, p.normalizedetg);
 #pragma unroll
     for (int v = 0; v < NRGPU_NV; ++v) out.p[v][x] = n[v];
   } else if (E.accmode == ACC_FINAL) {
@@ -1051,6 +913,29 @@ static int launch_bssn_tile(nrgpu_level *L, int b, const CUtensorMap *maps, cons
   return NRGPU_OK;
 }
 
+// The lists belong to the level: launches on them from several host
+// threads, or on several streams, take turns (the lock, and an event of the
+// last use; a stream that is being captured is ordered by its graph).
+struct ListTurn {
+  nrgpu_level *L;
+  cudaStream_t st;
+  bool capturing;
+  ListTurn(nrgpu_level *L_, cudaStream_t st_) : L(L_), st(st_) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    capturing = cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone;
+    // the lists are allocated here unless a graph is being captured (the
+    // refinement driver's first coarse step runs without one)
+    if (!capturing && L->parts) nrgpu_level_lists(L);
+    L->list_lock->lock();
+    if (L->lists && !capturing) cudaStreamWaitEvent(st, L->ev_lists, 0);
+  }
+  ~ListTurn() {
+    if (L->lists && !capturing) cudaEventRecord(L->ev_lists, st);
+    L->list_lock->unlock();
+  }
+  ListTurn(const ListTurn &) = delete;
+};
+
 // launch the interior and flagged kernels of one rhs evaluation
 // (kb <= k <= ke: the planes of the interior launch, whole boxes by default)
 static int launch_rhs(nrgpu_level *L, const CVarPtrs &U, const VarPtrs &out, const CVarPtrs &pre, const VarPtrs &acc,
@@ -1067,18 +952,16 @@ static int launch_rhs(nrgpu_level *L, const CVarPtrs &U, const VarPtrs &out, con
     NRGPU_CUDA_TRY(cudaStreamWaitEvent(L->side, L->ev_fork, 0));
   }
   if (interior) {
-    // the staging buffer of off-size boxes, allocated here unless a graph
-    // is being captured (the refinement driver allocates it beforehand)
-    if (!L->pad_tried) {
-      cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-      if (cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone) nrgpu_level_pad(L);
-      cudaGetLastError();
-    }
+    ListTurn turn(L, st);
     for (int b = 0; b < L->nboxes; ++b) {
       const BoxGeo &bx = L->hbox[b];
       if (bx.m < 3 || bx.n < 3 || bx.o < 3) continue;
       const int k0 = max(kb, 1), k1 = min(ke, bx.o - 2);
       if (k1 < k0) continue;
+      if (L->parts && !L->tile) {
+        if (p.order_centered == 4 && nrgpu_bssn_parts_o4(L, b, U.p, out.p, pre.p, acc.p, E, p, st, k0, k1)) continue;
+        if (p.order_centered == 6 && nrgpu_bssn_parts_o6(L, b, U.p, out.p, pre.p, acc.p, E, p, st, k0, k1)) continue;
+      }
       if (L->tile && tile_eligible(L, b, U.p, NRGPU_NV, p.order_centered, p.advection_lopsided,
                                    p.advection_lopsided6)) {
         const CUtensorMap *maps = nullptr;
@@ -1087,6 +970,9 @@ static int launch_rhs(nrgpu_level *L, const CVarPtrs &U, const VarPtrs &out, con
         if ((e = launch_bssn_tile(L, b, maps, U, out, pre, acc, E, p, st, k0, k1))) return e;
         continue;
       }
+      // point by point; the staging buffer of off-size boxes is allocated as
+      // the lists are
+      if (!turn.capturing) nrgpu_level_pad(L);
       // the block shape of the level (32 x 4 x 1, or what nrgpu_level_autotune
       // measured fastest for this box); 128 or 256 threads, one point each
       const dim3 blk(L->blk[0], L->blk[1], L->blk[2]);
@@ -1795,15 +1681,9 @@ static int z4_launch(nrgpu_level *L, const ZCVarPtrs &U, const ZVarPtrs &out, co
     NRGPU_CUDA_TRY(cudaStreamWaitEvent(L->side, L->ev_fork, 0));
   }
   if (interior) {
-    // the staging buffer of off-size boxes, allocated here unless a graph
-    // is being captured (the refinement driver allocates it beforehand)
-    if (!L->pad_tried) {
-      cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-      if (cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone) nrgpu_level_pad(L);
-      cudaGetLastError();
-    }
+    ListTurn turn(L, st);
     // all boxes in one persistent launch (nrgpu_level_queue), or one launch per box
-    const int qm = L->queue ? z4_queue_size(L, p) : 0;
+    const int qm = L->queue && !L->parts ? z4_queue_size(L, p) : 0;
     if (qm) {
       int e = z4_queue_launch(L, qm, U, out, pre, acc, E, p, st);
       if (e) return e;
@@ -1811,6 +1691,12 @@ static int z4_launch(nrgpu_level *L, const ZCVarPtrs &U, const ZVarPtrs &out, co
     for (int b = 0; b < L->nboxes && !qm; ++b) {
       const BoxGeo &bx = L->hbox[b];
       if (bx.m < 3 || bx.n < 3 || bx.o < 3) continue;
+      if (L->parts && p.precision == 0) {
+        const int k1 = bx.o - 2;
+        if (p.order_centered == 4 && nrgpu_z4_parts_o4(L, b, U.p, out.p, pre.p, acc.p, E, p, st, 1, k1)) continue;
+        if (p.order_centered == 6 && nrgpu_z4_parts_o6(L, b, U.p, out.p, pre.p, acc.p, E, p, st, 1, k1)) continue;
+      }
+      if (!turn.capturing) nrgpu_level_pad(L);
       // the block shape of the level (32 x 4 x 1, or what nrgpu_level_autotune
       // measured fastest for this box); 128 or 256 threads, one point each
       const dim3 blk(L->blk[0], L->blk[1], L->blk[2]);
@@ -1993,6 +1879,28 @@ extern "C" int nrgpu_level_autotune(nrgpu_level *L, int system, const void *para
                                 {64, 4, 1}, {32, 8, 1}, {16, 8, 2}, {32, 4, 2}, {16, 4, 4}, {8, 8, 4},
                                 {64, 2, 2}, {128, 2, 1}};
   const int ncand = (int)(sizeof cand / sizeof cand[0]);
+  // the two kernels of nrgpu_deriv.cuh take their tiles from the box: where
+  // they run, no shape is timed and the level's stays.  (They beat the
+  // staged tiles on every box: 66^3 0.21 against 0.27 ms.)
+  bool parts;
+  if (system == NRGPU_SYSTEM_BSSN) {
+    const nrgpu_bssn_params &q = *(const nrgpu_bssn_params *)params;
+    parts = nrgpu_parts_cover(q.order_centered, q.advection_lopsided, q.advection_lopsided6);
+  } else {
+    const nrgpu_z4_params &q = *(const nrgpu_z4_params *)params;
+    parts = q.precision == 0 && nrgpu_parts_cover(q.order_centered, q.advection_lopsided, q.advection_lopsided6);
+  }
+  for (int b = 0; b < L->nboxes; ++b)
+    parts = parts && (long)L->hbox[b].m * L->hbox[b].n * L->hbox[b].o >= 2 * NRGPU_PARTS_MIN_POINTS;
+  if (parts && L->parts && L->lists) {
+    L->tile = 0;
+    for (int q = 0; q < 3; ++q)
+      if (best_block) best_block[q] = L->blk[q];
+    cudaEventDestroy(ev0);
+    cudaEventDestroy(ev1);
+    NRGPU_CUDA_TRY(cudaStreamSynchronize(st));
+    return NRGPU_OK;
+  }
   float best = 1e30f;
   int bb = 0;
   for (int c = 0; c < ncand && !e; ++c) {

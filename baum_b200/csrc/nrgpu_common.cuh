@@ -20,6 +20,12 @@ struct CVarPtrs {
   const double *p[NRGPU_NV];
 };
 
+// NV device pointers to read from
+template <int NV>
+struct CPtrs {
+  const double *p[NV];
+};
+
 // device-side geometry of one box of a level
 struct BoxGeo {
   int m, n, o, noffset;

@@ -1,5 +1,6 @@
 // nrgpu_level.cuh -- device mirror of a BAM level (tL, bam_amr.h:46-74).
 #pragma once
+#include <mutex>
 #include "nrgpu_common.cuh"
 
 // one point with a non-zero boundary flag: linear index, box-local ijk,
@@ -17,6 +18,23 @@ struct FlagPoint {
 // parity under those reflections
 struct SymPoint {
   int dst, src, mask;
+};
+
+// how an rhs kernel leaves its results
+enum { EPI_RHS = 0, EPI_ADDLINEAR = 1, EPI_RK = 2 };
+
+// EPI_RK accumulator modes: ACC_ADD acc += wacc rhs; ACC_INIT acc = upre +
+// wacc rhs (the first stage, so that the step needs no copy of u); ACC_FINAL
+// out = acc + wacc rhs (the last stage writes u from the accumulator)
+enum { ACC_ADD = 0, ACC_INIT = 1, ACC_FINAL = 2 };
+
+struct Epilogue {
+  int mode;
+  double c;        // EPI_ADDLINEAR: unew = upre + c rhs
+  double wacc;     // EPI_RK: acc += wacc * rhs
+  double cv;       // EPI_RK: vout = upre + cv * rhs (when has_v)
+  int has_v;
+  int accmode;     // EPI_RK: ACC_ADD / ACC_INIT / ACC_FINAL
 };
 
 struct nrgpu_level {
@@ -43,6 +61,18 @@ struct nrgpu_level {
   double *pad;
   size_t pad_doubles;
   int pad_tried;
+  // 1: the interior rhs by the two kernels of nrgpu_deriv.cuh where they
+  // cover the run; 0: point by point (the levels of a deep hierarchy,
+  // nrgpu_fmr_create)
+  int parts;
+  // the lists of those kernels (first use): rows of
+  // NRGPU_DERIV_LISTS x NRGPU_DERIV_PITCH doubles; the lock and the event of
+  // their last use
+  double *lists;
+  size_t list_rows;
+  int lists_tried;
+  std::mutex *list_lock;
+  cudaEvent_t ev_lists;
   // device copy of a host state for the host-buffer entry points
   double *hoststate;
   // points with boundary flag 0, and the norm reduction buffer (first use)
@@ -106,6 +136,32 @@ inline int nrgpu_pad_size(int m, int n) {
   return 0;
 }
 void nrgpu_level_pad(nrgpu_level *L);
+// the lists of the two rhs kernels, allocated once per level; a level without
+// them runs the point-by-point kernels (nrgpu_lib.cu)
+#define NRGPU_DERIV_LISTS 71
+#define NRGPU_DERIV_PITCH 128
+#define NRGPU_PARTS_MIN_POINTS 50000
+#define NRGPU_PARTS_MAX_LEVELS 5
+void nrgpu_level_lists(nrgpu_level *L);
+// whether those kernels have the run's advection rows: shifts 1 and 2
+// (centred) at 4th order, 2 and 3 (centred) at 6th
+inline bool nrgpu_parts_cover(int order, int lop, int lop6) {
+  return order == 4 ? lop == 1 || lop == 2 : order == 6 && (lop6 == 2 || lop6 == 3);
+}
+// interior rhs of box b on planes kb .. ke by those kernels, per system and
+// order; false when they do not apply (nrgpu_parts_*.cu)
+bool nrgpu_bssn_parts_o4(nrgpu_level *L, int b, const double *const *U, double *const *out, const double *const *pre,
+                         double *const *acc, const Epilogue &E, const nrgpu_bssn_params &p, cudaStream_t st, int kb,
+                         int ke);
+bool nrgpu_bssn_parts_o6(nrgpu_level *L, int b, const double *const *U, double *const *out, const double *const *pre,
+                         double *const *acc, const Epilogue &E, const nrgpu_bssn_params &p, cudaStream_t st, int kb,
+                         int ke);
+bool nrgpu_z4_parts_o4(nrgpu_level *L, int b, const double *const *U, double *const *out, const double *const *pre,
+                       double *const *acc, const Epilogue &E, const nrgpu_z4_params &p, cudaStream_t st, int kb,
+                       int ke);
+bool nrgpu_z4_parts_o6(nrgpu_level *L, int b, const double *const *U, double *const *out, const double *const *pre,
+                       double *const *acc, const Epilogue &E, const nrgpu_z4_params &p, cudaStream_t st, int kb,
+                       int ke);
 // set_boundary_symmetry on a list of nv variables of the given system
 // (NRGPU_SYSTEM_BSSN / _Z4C); nothing without symmetry (nrgpu_bssn.cu)
 int nrgpu_level_symmetry(nrgpu_level *L, double *const *u, int system, cudaStream_t st);

@@ -4,6 +4,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <new>
 #include <vector>
 #include "nrgpu_level.cuh"
 
@@ -143,6 +144,11 @@ extern "C" int nrgpu_level_create(const nrgpu_level_desc *d, nrgpu_level **out) 
   }
   nrgpu_level *L = (nrgpu_level *)calloc(1, sizeof(nrgpu_level));
   if (!L) return nrgpu_set_error(NRGPU_ERR_NOMEM, "host allocation");
+  L->list_lock = new (std::nothrow) std::mutex;
+  if (!L->list_lock) {
+    free(L);
+    return nrgpu_set_error(NRGPU_ERR_NOMEM, "host allocation");
+  }
   cudaGetDevice(&L->device);
   L->nboxes = d->nboxes;
   L->npoints = d->npoints;
@@ -155,6 +161,7 @@ extern "C" int nrgpu_level_create(const nrgpu_level_desc *d, nrgpu_level **out) 
   for (int q = 0; q < 3; ++q) L->nladder[q] = nlad[q];
   L->ninner = (long)d->npoints - (long)fl.size();
   L->blk[0] = 32; L->blk[1] = 4; L->blk[2] = 1;
+  L->parts = 1;
   if (cudaDeviceGetAttribute(&L->nsm, cudaDevAttrMultiProcessorCount, L->device) != cudaSuccess || L->nsm < 1)
     L->nsm = 148;
   L->symmetry = d->symmetry;
@@ -194,6 +201,9 @@ extern "C" int nrgpu_level_destroy(nrgpu_level *L) {
   cudaFree(L->rsym);
   cudaFree(L->scratch);
   cudaFree(L->pad);
+  cudaFree(L->lists);
+  if (L->ev_lists) cudaEventDestroy(L->ev_lists);
+  delete L->list_lock;
   cudaFree(L->hoststate);
   cudaFree(L->d_red);
   cudaFree(L->d_red0d);
@@ -212,8 +222,6 @@ extern "C" int nrgpu_level_destroy(nrgpu_level *L) {
   return NRGPU_OK;
 }
 
-// three variable lists of RK4 scratch (room for the 25 Z4c variables),
-// allocated once per level
 // the staging buffer for boxes of up to 194 points per side without a
 // compile-time-stride kernel of their own: 25 lists with strides (1, P, P P),
 // P the next kernel size (kPadSizes); tried once per level, and a level
@@ -235,6 +243,31 @@ void nrgpu_level_pad(nrgpu_level *L) {
   }
 }
 
+// The lists that the two rhs kernels pass from one to the other, for as many
+// rows of a part of the largest box as kListBytes hold.
+constexpr size_t kListBytes = (size_t)512 << 20;
+void nrgpu_level_lists(nrgpu_level *L) {
+  std::lock_guard<std::mutex> g(*L->list_lock);
+  if (L->lists_tried) return;
+  L->lists_tried = 1;
+  constexpr size_t row = sizeof(double) * NRGPU_DERIV_LISTS * NRGPU_DERIV_PITCH;
+  size_t rows = 0;
+  for (int b = 0; b < L->nboxes; ++b)
+    if ((long)L->hbox[b].m * L->hbox[b].n * L->hbox[b].o >= NRGPU_PARTS_MIN_POINTS)
+      rows = std::max(rows, (size_t)L->hbox[b].n * std::max(0, L->hbox[b].o - 4));
+  rows = std::min(rows, kListBytes / row);
+  if (rows && cudaMalloc(&L->lists, rows * row) == cudaSuccess &&
+      cudaEventCreateWithFlags(&L->ev_lists, cudaEventDisableTiming) == cudaSuccess) {
+    L->list_rows = rows;
+  } else {
+    cudaGetLastError();
+    cudaFree(L->lists);
+    L->lists = nullptr;
+  }
+}
+
+// three variable lists of RK4 scratch (room for the 25 Z4c variables),
+// allocated once per level
 int nrgpu_level_scratch(nrgpu_level *L, double **out) {
   if (!L->scratch) {
     const size_t bytes = sizeof(double) * 3 * NRGPU_Z4_NVARS * (size_t)L->npoints;
@@ -244,7 +277,8 @@ int nrgpu_level_scratch(nrgpu_level *L, double **out) {
       return nrgpu_set_error(NRGPU_ERR_NOMEM, "RK4 scratch of %zu bytes", bytes);
     }
     L->scratch_points = (size_t)L->npoints;
-    nrgpu_level_pad(L);
+    if (L->parts) nrgpu_level_lists(L);
+    if (!L->lists) nrgpu_level_pad(L);
   }
   *out = L->scratch;
   return NRGPU_OK;

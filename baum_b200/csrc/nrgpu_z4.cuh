@@ -11,9 +11,6 @@
 // one thread computes one inner point, derivative groups are consumed as
 // soon as they are formed, and advection/dissipation are added last.
 
-enum { ZG11 = 0, ZCHI = 6, ZA11 = 7, ZKHAT = 13, ZGA1 = 14, ZTHETA = 17, ZALPHA = 18, ZBETA1 = 19, ZBB1 = 22 };
-constexpr int ZNV = NRGPU_Z4_NVARS;
-
 struct ZVarPtrs {
   double *p[ZNV];
 };
@@ -384,10 +381,7 @@ __device__ __forceinline__ void z4_store(const double r[ZNV], int x, const ZVarP
     double n[ZNV];
 #pragma unroll
     for (int v = 0; v < ZNV; ++v) n[v] = ldg(pre.p[v] + x) + E.c * r[v];
-    nrgpu_bssn_params q;  // only subtractA / normalizedetg are read
-    q.subtractA = p.subtractA;
-    q.normalizedetg = p.normalizedetg;
-    det_trace_fix(n, q);  // g~ at 0..5 and A~ at 7..12 in both lists
+    det_trace_fix(n, p.subtractA, p.normalizedetg);
 #pragma unroll
     for (int v = 0; v < ZNV; ++v) out.p[v][x] = n[v];
   } else if (E.accmode == ACC_FINAL) {

@@ -494,7 +494,12 @@ int nrgpu_psi4_modes(nrgpu_level *L, const double *rpsi4, const double *ipsi4, c
 enum { NRGPU_SYSTEM_BSSN = 0, NRGPU_SYSTEM_Z4C = 1 };
 
 /* ---- launch-shape autotuner (no counterpart in the reference) -------------
- * The rhs kernels compute one point per thread in blocks of 128 or 256
+ * Boxes of at least 50000 inner points run their 4th- and 6th-order interior
+ * rhs in two kernels that choose their own tiles (advection shifts 1 and 2 at
+ * 4th order, 2 and 3 at 6th; FP64; not on the levels of a hierarchy deeper
+ * than five): there nothing is timed and the level's shape stays.  Their
+ * intermediate lists take up to 512 MB per level, allocated on first use.
+ * The other rhs kernels compute one point per thread in blocks of 128 or 256
  * threads.  nrgpu_level_autotune times twenty block shapes (x, y, z
  * extents, from 32 x 4 x 1 and 8 x 16 x 1 to 8 x 4 x 4, 16 x 8 x 2 and
  * 8 x 8 x 4) for the level's boxes
@@ -522,9 +527,10 @@ int nrgpu_level_tile(nrgpu_level *L, int on);
 /* The Z4c interior rhs of all boxes of a level in one persistent launch:
  * the blocks take tiles from a queue over the boxes (an atomic counter)
  * until it is empty, each point computed as by the per-box kernel, so the
- * results are identical.  For levels of two or more boxes of one size that
- * has a compile-time-stride kernel (66, 72, 104, 136, 162, 168, 194 points
- * in x and y), 4th or 6th order, FP64; one launch per box otherwise.
+ * results are identical.  For levels of a hierarchy deeper than five that
+ * have two or more boxes of one size with a compile-time-stride kernel (66,
+ * 72, 104, 136, 162, 168, 194 points in x and y), 4th or 6th order, FP64; one
+ * launch per box otherwise.
  * on = 1 on, 0 off, -1 only queries; returns the setting.
  * nrgpu_level_autotune turns it on where it measures faster.  No
  * counterpart in the reference (advance_levelandsublevels, main.c:397-418,

@@ -1,0 +1,97 @@
+"""The two-kernel interior rhs (nrgpu_deriv.cuh) against the CPU oracle, at
+the sizes where its cutting can go wrong: a row of exactly one part (120
+interior points), one point more (two parts), three parts, few planes, tiles
+with a remainder in both directions; both systems and orders, the upwind rows
+it has (and one it has not), 4th-order dissipation and none, the B equation
+without the advection of Gamma~, and the add-linear form.  Tolerance: 1e-12 of
+each field's largest rhs, as for the other rhs kernels (second differences of
+a field of 1 at dx 0.3 round to ~30 eps / dx^2 = 7e-14)."""
+import numpy as np
+import pytest
+import torch
+
+from baum_b200 import abi, bssn, synthetic, z4
+from conftest import relerr
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-12
+
+
+def box(m, n, o, dx=0.3):
+    b = np.zeros((o, n, m), dtype=np.int32)
+    b[0], b[-1], b[:, 0], b[:, -1], b[:, :, 0], b[:, :, -1] = (abi.PHYBOUND,) * 6
+    return abi.Level([(m, n, o, -0.5 * (m - 1) * dx + 0.01, -0.5 * (n - 1) * dx, -0.5 * (o - 1) * dx)], dx, b.ravel())
+
+
+def state(lev, system):
+    x, y, z = lev.coords()
+    nv, unit = (abi.NVARS, synthetic.BSSN_UNIT) if system == "bssn" else (abi.Z4_NVARS, synthetic.Z4_UNIT)
+    u = synthetic.fourier_state(x, y, z, nv, unit, 8, 0.02, 9.0, 7)
+    b = nv - 6
+    u[b] += 0.1 * np.sin(0.3 * y)      # both signs of the shift in every direction
+    u[b + 1] -= 0.1 * np.cos(0.2 * x)
+    u[b + 2] += 0.1 * np.sin(0.4 * z)
+    return u
+
+
+@pytest.mark.parametrize("system,shape,order,over", [
+    ("bssn", (124, 28, 26), 4, {}),                                  # 120 x 24 x 22 inner: one part wide
+    ("z4", (125, 28, 26), 4, {}),                                    # 121: two parts
+    ("z4", (247, 23, 19), 6, {}),                                    # 241 x 17 x 13 inner: three parts
+    ("bssn", (101, 103, 11), 4, {}),                                 # few planes
+    ("bssn", (47, 43, 41), 6, {"advection_lopsided6": 2}),
+    ("z4", (47, 43, 41), 6, {"advection_lopsided6": 2, "order_dissipation": 4, "dissfactor": 0.1 / 16}),
+    ("bssn", (47, 43, 41), 4, {"order_dissipation": 4, "dissfactor": 0.1 / 16}),
+    ("z4", (47, 43, 41), 4, {"advection_lopsided": 2, "order_dissipation": 0}),
+    ("bssn", (47, 43, 41), 4, {"withGadv": 0.0}),
+    ("z4", (47, 43, 41), 4, {"withGadv": 0.0, "shiftalphapower": 0.5, "chipsipower": -2.0}),
+    ("bssn", (47, 43, 41), 4, {"advection_lopsided": 0}),            # point by point
+])
+def test_two_kernel_rhs_matches_oracle(gpu, system, shape, order, over):
+    lev = box(*shape)
+    u0 = state(lev, system)
+    kw = dict(order_centered=order, order_advection=order, **over)
+    mod, p, ref = (bssn, abi.bssn_params(**kw), oracle.bssn_rhs) if system == "bssn" else \
+        (z4, abi.z4_params(**kw), oracle.z4_rhs)
+    dl = mod.DeviceLevel(lev)
+    nv = u0.shape[0]
+    u, r = torch.from_numpy(u0).cuda(), dl.empty(nv)
+    mod.evolve_rhs(dl, r, u, 0.0, u, p)
+    n = torch.from_numpy(u0.copy()).cuda()
+    mod.evolve_rhs(dl, n, n, 0.01, u, p)        # add-linear, in place on the previous state
+    torch.cuda.synchronize()
+    assert not dl.nan_flag()
+    ro = ref(lev, u0, p)
+    e = relerr(r.cpu().numpy(), ro)
+    assert e.max() < TOL, e
+    no = ref(lev, u0, p, c=0.01, upre=u0)
+    e = relerr(n.cpu().numpy(), no)
+    assert e.max() < TOL, e
+    dl.close()
+
+
+def test_two_streams_share_the_lists(gpu):
+    """rhs calls of one level on two streams, different states, interleaved:
+    each equals its own serial result bit for bit."""
+    lev = box(60, 52, 44)
+    p = abi.z4_params()
+    dl = z4.DeviceLevel(lev)
+    us = [torch.from_numpy(state(lev, "z4") * f).cuda() for f in (1.0, 1.001)]
+    serial = []
+    for u in us:
+        r = dl.empty(25)
+        z4.z4_rhs_movpunc_N(dl, r, u, 0.0, u, p)
+        torch.cuda.synchronize()
+        serial.append(r)
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    rs = [[dl.empty(25) for _ in range(4)] for _ in us]
+    torch.cuda.synchronize()
+    for k in range(4):
+        for u, r, s in zip(us, rs, streams):
+            z4.z4_rhs_movpunc_N(dl, r[k], u, 0.0, u, p, s)
+    torch.cuda.synchronize()
+    for want, got in zip(serial, rs):
+        for g in got:
+            assert torch.equal(want, g)
+    dl.close()
