@@ -33,8 +33,10 @@ struct ConfIn {
 __global__ void to_adm_kernel(ConfIn u, AdmOut adm, double oochipsipower, int np) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= np) return;
-  const double psi = pow(ldg(u.p[6] + i), oochipsipower);
-  const double psi4 = pow(psi, 4.0);
+  // psi^4 = chi^(4 / p): 1 / chi for the usual p = -4 (NaN for a negative chi,
+  // as the power gives)
+  const double chi = ldg(u.p[6] + i);
+  const double psi4 = oochipsipower == -0.25 ? (chi < 0.0 ? nan("") : 1.0 / fabs(chi)) : pow(pow(chi, oochipsipower), 4.0);
   const double trK = ldg(u.p[13] + i);
 #pragma unroll
   for (int n = 0; n < 6; ++n) {
@@ -216,12 +218,237 @@ __device__ __forceinline__ int ladder_c(int order, int d) {
   return 6;
 }
 
-// one thread per point of the box interior; flag-0 points only
-// (forinnerpoints_ijk, bam_amr_loops_box.h:138)
+// ---- constraints of the points with room for the full stencils --------------------
+// One 32 x 8 tile of a plane per block.  Per metric component each thread
+// takes the derivatives along the axes from its own 6 ORD / 2 + 1 taps and
+// leaves d_y g and d_z g in shared memory, with ORD / 2 columns and rows
+// around the tile; the mixed second derivatives are d_x (d_y g), d_x (d_z g),
+// d_y (d_z g) from there (product stencils, discretize.m:68-71): 28 loads per
+// component and point instead of 61 at 4th order.  The second derivatives
+// enter the Ricci scalar with one weight each, so none is kept:
+//   R = [ g^ab g^cd - g^bd g^ac ] d_a d_c g_bd + Gamma^e_ac Gamma_e^ac
+//       - Gamma^e Gamma_e,
+//   mom_a = g^bc (d_c K_ab - d_a K_bc) + Gamma^d_ab K^b_d - Gamma^d K_ad
+// (the sums of adm_constraints_N.m contracted pairwise; MODE 1 keeps
+// D^c K_ac and g^bc D_a K_bc apart for its denominators).  With every order in
+// one kernel, all 36 second derivatives in registers and the sums term by
+// term, a 104^3 box took 0.79 ms (variables, constraints and norms); so, it
+// takes 0.41 ms, 0.27 of them in this kernel.  What bounds it is latency at 8 to
+// 16 warps per SM.  Two blocks per SM leave 128 registers: at 2nd order they hold
+// everything (104^3: 0.28 against 0.31 ms with one block), above it 300 bytes
+// spill (4th order 0.424 against 0.413, 66^3 at 6th 0.199 against 0.177).
+constexpr int kCX = 32, kCY = 8;
+
+template <int ORD, int MODE>
+__global__ void __launch_bounds__(kCX *kCY, ORD == 2 ? 2 : 1) adm_constraints_tile_kernel(AdmIn A, ConOut C, BoxGeo box,
+                                                                        const int *__restrict__ boundary, double dx,
+                                                                        double dy, double dz, int *status) {
+  constexpr int H = ORD / 2;
+  __shared__ double DY[2][kCY][kCX + 2 * H], DZ[2][kCY + 2 * H][kCX + 2 * H];
+  const int tx = threadIdx.x, ty = threadIdx.y, t = ty * kCX + tx;
+  const int i0 = H + blockIdx.x * kCX, j0 = H + blockIdx.y * kCY, k = H + blockIdx.z;
+  // threads beyond the interior store no constraints; their d_y g and d_z g are
+  // taps of the points beside them (xy, xz: their own column and row as far as
+  // the box and the stencil go)
+  const bool mine = i0 + tx < box.m - H && j0 + ty < box.n - H;
+  const int i = min(i0 + tx, box.m - 1 - H), j = min(j0 + ty, box.n - 1 - H);
+  const int st[3] = {1, box.m, box.m * box.n};
+  const int x = box.noffset + i + box.m * (j + box.n * k);
+  const int ie = min(i0 + tx, box.m - 1), xy = box.noffset + ie + box.m * (j + box.n * k);
+  const int xz = box.noffset + ie + box.m * (min(j0 + ty, box.n - 1) + box.n * k);
+  const double i1[3] = {1.0 / (den1<ORD>() * dx), 1.0 / (den1<ORD>() * dy), 1.0 / (den1<ORD>() * dz)};
+  const double i2[6] = {1.0 / (den2<ORD>() * dx * dx), i1[0] * i1[1], i1[0] * i1[2],
+                        1.0 / (den2<ORD>() * dy * dy), i1[1] * i1[2], 1.0 / (den2<ORD>() * dz * dz)};
+  // one point of the frame of DZ (columns left and right of the tile, rows
+  // above and below), and of DY (columns)
+  int zx = -1, zr = 0, zc = 0, yx = -1, yr = 0, yc = 0;
+  if (t < (kCX + kCY) * 2 * H) {
+    if (t < kCY * 2 * H) {
+      const int q = t % (2 * H);
+      zr = t / (2 * H);
+      zc = q < H ? q - H : kCX + q - H;
+    } else {
+      const int u = t - kCY * 2 * H, q = u / kCX;
+      zc = u % kCX;
+      zr = q < H ? q - H : kCY + q - H;
+    }
+    zx = box.noffset + min(i0 + zc, box.m - 1) + box.m * (min(j0 + zr, box.n - 1) + box.n * k);
+  }
+  if (t < kCY * 2 * H) {
+    const int q = t % (2 * H);
+    yr = t / (2 * H);
+    yc = q < H ? q - H : kCX + q - H;
+    yx = box.noffset + min(i0 + yc, box.m - 1) + box.m * (min(j0 + yr, box.n - 1 - H) + box.n * k);
+  }
+  double g[6], gi[6], dg[3][6];
+#pragma unroll
+  for (int v = 0; v < 6; ++v) g[v] = ldg(A.p[v] + x);
+  {
+    const double det = g[0] * (g[3] * g[5] - g[4] * g[4]) - g[1] * (g[1] * g[5] - g[2] * g[4]) +
+                       g[2] * (g[1] * g[4] - g[2] * g[3]);
+    const double idet = 1.0 / det;
+    gi[0] = (g[3] * g[5] - g[4] * g[4]) * idet;
+    gi[1] = (g[2] * g[4] - g[1] * g[5]) * idet;
+    gi[2] = (g[1] * g[4] - g[2] * g[3]) * idet;
+    gi[3] = (g[0] * g[5] - g[2] * g[2]) * idet;
+    gi[4] = (g[1] * g[2] - g[0] * g[4]) * idet;
+    gi[5] = (g[0] * g[3] - g[1] * g[1]) * idet;
+  }
+  double R = 0.0;
+#pragma unroll
+  for (int b = 0; b < 3; ++b)
+#pragma unroll
+    for (int d = b; d < 3; ++d) {
+      const int v = sy(b, d);
+      const double *f = A.p[v];
+      double n1[3], n2[6];
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        n1[a] = d1n<ORD>(f, a == 0 ? x : a == 1 ? xy : xz, st[a]);
+        n2[sy(a, a)] = d2n<ORD>(f, x, st[a]);
+      }
+      double (*const Y)[kCX + 2 * H] = DY[v & 1], (*const Z)[kCX + 2 * H] = DZ[v & 1];
+      Y[ty][tx + H] = n1[1];
+      Z[ty + H][tx + H] = n1[2];
+      if (zx >= 0) Z[zr + H][zc + H] = d1n<ORD>(f, zx, st[2]);
+      if (yx >= 0) Y[yr][yc + H] = d1n<ORD>(f, yx, st[1]);
+      __syncthreads();  // (the buffer after next is written after the next barrier)
+      auto num = [](const double *c, int s) {
+        if (ORD == 2) return c[s] - c[-s];
+        if (ORD == 4) return (c[-2 * s] - c[2 * s]) + 8.0 * (c[s] - c[-s]);
+        return (c[3 * s] - c[-3 * s]) + 9.0 * (c[-2 * s] - c[2 * s]) + 45.0 * (c[s] - c[-s]);
+      };
+      n2[1] = num(&Y[ty][tx + H], 1);
+      n2[2] = num(&Z[ty + H][tx + H], 1);
+      n2[4] = num(&Z[ty + H][tx + H], kCX + 2 * H);
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        dg[a][v] = i1[a] * n1[a];
+#pragma unroll
+        for (int c = a; c < 3; ++c) {
+          // both orders of (a, c), and of (b, d)
+          const double w = 0.5 * (gi[sy(a, b)] * gi[sy(c, d)] + gi[sy(c, b)] * gi[sy(a, d)]) - gi[v] * gi[sy(a, c)];
+          R += ((a == c ? 1.0 : 2.0) * (b == d ? 1.0 : 2.0)) * w * (i2[sy(a, c)] * n2[sy(a, c)]);
+        }
+      }
+    }
+  if (!mine || __ldg(boundary + x) != 0) return;
+  double gd[3][6], gu[3][6], Gu[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c)
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+      for (int b = a; b < 3; ++b) gd[c][sy(a, b)] = 0.5 * (dg[a][sy(b, c)] + dg[b][sy(a, c)] - dg[c][sy(a, b)]);
+#pragma unroll
+  for (int c = 0; c < 3; ++c)
+#pragma unroll
+    for (int q = 0; q < 6; ++q) gu[c][q] = gi[sy(c, 0)] * gd[0][q] + gi[sy(c, 1)] * gd[1][q] + gi[sy(c, 2)] * gd[2][q];
+  auto trace = [&](const double q[6]) {
+    return gi[0] * q[0] + gi[3] * q[3] + gi[5] * q[5] + 2.0 * (gi[1] * q[1] + gi[2] * q[2] + gi[4] * q[4]);
+  };
+#pragma unroll
+  for (int e = 0; e < 3; ++e) {
+    Gu[e] = trace(gu[e]);
+    R -= Gu[e] * trace(gd[e]);
+    // Gamma^e_ac Gamma_e^ac
+    double m[3][3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+      for (int b = 0; b < 3; ++b)
+        m[a][b] = gi[sy(a, 0)] * gd[e][sy(0, b)] + gi[sy(a, 1)] * gd[e][sy(1, b)] + gi[sy(a, 2)] * gd[e][sy(2, b)];
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+      for (int c = a; c < 3; ++c)
+        R += (a == c ? 1.0 : 2.0) * gu[e][sy(a, c)] *
+             (m[a][0] * gi[sy(0, c)] + m[a][1] * gi[sy(1, c)] + m[a][2] * gi[sy(2, c)]);
+  }
+  double K[6], Kud[3][3];
+#pragma unroll
+  for (int v = 0; v < 6; ++v) K[v] = ldg(A.p[6 + v] + x);
+#pragma unroll
+  for (int a = 0; a < 3; ++a)
+#pragma unroll
+    for (int b = 0; b < 3; ++b)
+      Kud[a][b] = gi[sy(a, 0)] * K[sy(0, b)] + gi[sy(a, 1)] * K[sy(1, b)] + gi[sy(a, 2)] * K[sy(2, b)];
+  const double trK = Kud[0][0] + Kud[1][1] + Kud[2][2];
+  double KK = 0.0, s1[3], s2[3];  // s1 = D^c K_ac, s2 = g^bc D_a K_bc
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    s1[a] = s2[a] = 0.0;
+#pragma unroll
+    for (int b = 0; b < 3; ++b) {
+      KK += Kud[a][b] * Kud[b][a];
+      s1[a] -= Gu[b] * K[sy(a, b)];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        const double q = gu[d][sy(a, b)] * Kud[b][d];
+        s1[a] -= q;
+        s2[a] -= 2.0 * q;
+      }
+    }
+  }
+#pragma unroll
+  for (int b = 0; b < 3; ++b)
+#pragma unroll
+    for (int c = b; c < 3; ++c) {
+      const int v = sy(b, c);
+      double dK[3];
+#pragma unroll
+      for (int a = 0; a < 3; ++a) dK[a] = i1[a] * d1n<ORD>(A.p[6 + v], x, st[a]);
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        s2[a] += (b == c ? 1.0 : 2.0) * gi[v] * dK[a];
+        s1[b] += gi[sy(a, c)] * dK[a];
+        if (b != c) s1[c] += gi[sy(a, b)] * dK[a];
+      }
+    }
+  double out[8];
+  out[0] = R + trK * trK - KK;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) out[1 + a] = s1[a] - s2[a];
+  if (MODE == 1) {
+    double den = fabs(R) + trK * trK + fabs(KK);
+    out[4] = den <= 0.0 ? 0.0 : out[0] / den;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      den = fabs(s1[a]) + fabs(s2[a]);
+      out[5 + a] = den <= 0.0 ? 0.0 : out[1 + a] / den;
+    }
+  }
+  if (!isfinite(out[0])) atomicOr(status, 1);
+#pragma unroll
+  for (int v = 0; v < (MODE ? 8 : 4); ++v) C.p[v][x] = out[v];
+}
+
+// the points nearer the faces, at the orders that fit there (the level's
+// ladder list)
 template <int MODE>
-__global__ void __launch_bounds__(128) adm_constraints_kernel(AdmIn A, ConOut C, BoxGeo box,
-                                                             const int *__restrict__ boundary, int order,
-                                                             double dx, double dy, double dz, int *status) {
+__global__ void __launch_bounds__(128) adm_constraints_ladder_kernel(AdmIn A, ConOut C, const FlagPoint *__restrict__ pts,
+                                                                     int n, const BoxGeo *__restrict__ boxes, int order,
+                                                                     double dx, double dy, double dz, int *status) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n) return;
+  const FlagPoint fp = pts[t];
+  if (fp.flag == 0) return;  // a flag-0 point on a face has no stencil
+  const BoxGeo b = boxes[fp.box];
+  const int st[3] = {1, b.m, b.m * b.n};
+  const double h[3] = {dx, dy, dz};
+  double out[8];
+  if (ladder_c(order, fp.flag) == 2) con_point<2, MODE>(A, fp.ijk, st, h, out);
+  else con_point<4, MODE>(A, fp.ijk, st, h, out);
+  if (!isfinite(out[0])) atomicOr(status, 1);
+#pragma unroll
+  for (int v = 0; v < (MODE ? 8 : 4); ++v) C.p[v][fp.ijk] = out[v];
+}
+
+// term by term: one thread per point of the box interior; flag-0 points only
+// (forinnerpoints_ijk, bam_amr_loops_box.h:138)
+__global__ void __launch_bounds__(128) adm_constraints_terms_kernel(AdmIn A, ConOut C, BoxGeo box,
+                                                                   const int *__restrict__ boundary, int order,
+                                                                   double dx, double dy, double dz, int *status) {
   const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
   const int j = 1 + blockIdx.y * blockDim.y + threadIdx.y;
   const int k = 1 + blockIdx.z;
@@ -234,13 +461,12 @@ __global__ void __launch_bounds__(128) adm_constraints_kernel(AdmIn A, ConOut C,
   const double h[3] = {dx, dy, dz};
   double out[8];
   const int ord = ladder_c(order, d);
-  if (ord == 2) con_point<2, MODE>(A, x, st, h, out);
-  else if (ord == 4) con_point<4, MODE>(A, x, st, h, out);
-  else con_point<6, MODE>(A, x, st, h, out);
+  if (ord == 2) con_point<2, 2>(A, x, st, h, out);
+  else if (ord == 4) con_point<4, 2>(A, x, st, h, out);
+  else con_point<6, 2>(A, x, st, h, out);
   if (!isfinite(out[0])) atomicOr(status, 1);
-  const int nout = MODE ? 8 : 4;
 #pragma unroll
-  for (int v = 0; v < nout; ++v) C.p[v][x] = out[v];
+  for (int v = 0; v < 8; ++v) C.p[v][x] = out[v];
 }
 
 // ---- norms ------------------------------------------------------------------
@@ -324,6 +550,28 @@ extern "C" int nrgpu_to_adm(nrgpu_level *L, const double *const *u, double *cons
   return NRGPU_OK;
 }
 
+template <int MODE>
+static void launch_constraints(nrgpu_level *L, const AdmIn &A, const ConOut &C, int order, cudaStream_t st) {
+  const int H = order / 2;
+  for (int b = 0; b < L->nboxes; ++b) {
+    const BoxGeo &bx = L->hbox[b];
+    if (bx.m <= 2 * H || bx.n <= 2 * H || bx.o <= 2 * H) continue;
+    const dim3 blk(kCX, kCY, 1);
+    const dim3 grd((bx.m - 2 * H + kCX - 1) / kCX, (bx.n - 2 * H + kCY - 1) / kCY, bx.o - 2 * H);
+#define NR_CON(ORD_)                                                                                              \
+  adm_constraints_tile_kernel<ORD_, MODE><<<grd, blk, 0, st>>>(A, C, bx, L->d_boundary, L->dx, L->dy, L->dz, \
+                                                               L->d_status)
+    if (order == 2) NR_CON(2);
+    else if (order == 4) NR_CON(4);
+    else NR_CON(6);
+#undef NR_CON
+  }
+  const int n = L->nladder[H - 1];
+  if (n > 0)
+    adm_constraints_ladder_kernel<MODE><<<(n + 127) / 128, 128, 0, st>>>(A, C, L->d_ladder, n, L->d_box, order, L->dx,
+                                                                         L->dy, L->dz, L->d_status);
+}
+
 extern "C" int nrgpu_adm_constraints(nrgpu_level *L, const double *const *adm, double *const *con,
                                      int order_centered, int mode, void *stream) {
   if (!L || !adm || !con) return nrgpu_set_error(NRGPU_ERR_ARG, "null argument");
@@ -344,22 +592,22 @@ extern "C" int nrgpu_adm_constraints(nrgpu_level *L, const double *const *adm, d
   }
   NRGPU_CUDA_TRY(cudaSetDevice(L->device));
   const cudaStream_t st = (cudaStream_t)stream;
-  for (int b = 0; b < L->nboxes; ++b) {
-    const BoxGeo &bx = L->hbox[b];
-    if (bx.m < 3 || bx.n < 3 || bx.o < 3) continue;
-    const dim3 blk(32, 4, 1);
-    const dim3 grd((bx.m - 2 + 31) / 32, (bx.n - 2 + 3) / 4, bx.o - 2);
-    if (mode == NRGPU_CON_PLAIN)
-      adm_constraints_kernel<0><<<grd, blk, 0, st>>>(A, C, bx, L->d_boundary, order_centered, L->dx, L->dy,
-                                                     L->dz, L->d_status);
-    else if (mode == NRGPU_CON_NORMALIZED)
-      adm_constraints_kernel<1><<<grd, blk, 0, st>>>(A, C, bx, L->d_boundary, order_centered, L->dx, L->dy,
-                                                     L->dz, L->d_status);
-    else
-      adm_constraints_kernel<2><<<grd, blk, 0, st>>>(A, C, bx, L->d_boundary, order_centered, L->dx, L->dy,
-                                                     L->dz, L->d_status);
-    NRGPU_CUDA_TRY(cudaGetLastError());
+  // term by term, in the generated code's order, for every point; else the
+  // tiles, and the points near the faces from the level's list
+  if (mode == NRGPU_CON_TERMBYTERM) {
+    for (int b = 0; b < L->nboxes; ++b) {
+      const BoxGeo &bx = L->hbox[b];
+      if (bx.m < 3 || bx.n < 3 || bx.o < 3) continue;
+      const dim3 blk(32, 4, 1), grd((bx.m - 2 + 31) / 32, (bx.n - 2 + 3) / 4, bx.o - 2);
+      adm_constraints_terms_kernel<<<grd, blk, 0, st>>>(A, C, bx, L->d_boundary, order_centered, L->dx, L->dy, L->dz,
+                                                     L->d_status);
+    }
+  } else if (mode == NRGPU_CON_PLAIN) {
+    launch_constraints<0>(L, A, C, order_centered, st);
+  } else {
+    launch_constraints<1>(L, A, C, order_centered, st);
   }
+  NRGPU_CUDA_TRY(cudaGetLastError());
   return NRGPU_OK;
 }
 

@@ -66,6 +66,35 @@ def test_constraints_match_oracle_on_puncture(gpu, order, mode):
     check_constraints(con.cpu().numpy()[:, inner], co[:, inner])
 
 
+@pytest.mark.parametrize("order", [2, 4, 6])
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("shape", [(9, 8, 7), (38, 20, 9), (41, 31, 10), (71, 22, 13)])
+def test_constraint_tiles_match_oracle(gpu, shape, order, mode):
+    """The 32 x 8 tiles at their edges: boxes of one part of a tile, of 32
+    inner columns at order 6, of one tile and a remainder in each direction,
+    with the ladder of lower orders around; one flagged point inside,
+    and a metric with no symmetry."""
+    m, n, o = shape
+    b = np.zeros((o, n, m), dtype=np.int32)
+    b[0], b[-1], b[:, 0], b[:, -1], b[:, :, 0], b[:, :, -1] = (abi.PHYBOUND,) * 6
+    b[o // 2, n // 2, m // 2] = abi.PHYBOUND
+    lev = abi.Level([(m, n, o, -3.0, -2.0, -1.0)], 0.3, b.ravel())
+    rng = np.random.default_rng(m + order)
+    u = 0.1 * rng.standard_normal((12, lev.npoints))
+    u[[0, 3, 5]] += 1.0
+    dl = bssn.DeviceLevel(lev)
+    con = dl.empty(8 if mode else 4)
+    con.zero_()
+    adm.adm_constraints_N(dl, con, to_dev(u), order, mode)
+    co = oracle.adm_constraints(lev, u, order, mode)
+    out = con.cpu().numpy()
+    inner = lev.boundary == 0
+    assert (out[:, ~inner] == 0).all()
+    # the sums reach their largest terms at the point of the largest
+    # constraint: 1e-12 of it is > 1000 eps of any term
+    check_constraints(out[:, inner], co[:, inner], 1e-12)
+
+
 def test_norms_match_oracle(gpu):
     g = load_golden("bssn_punc_con")
     lev = golden_level(g)
