@@ -1,6 +1,5 @@
 // nrgpu_algebra.cuh -- the BSSN and Z4c right-hand sides at one point, from
-// derivatives that a source provides (included inside the anonymous
-// namespace of nrgpu_bssn.cu).
+// derivatives that a source provides (included by nrgpu_parts.cuh).
 //
 // The physics is bssn_rhs_movpunc_N (spec bssn_rhs_movpunc_N.m:218-372) and
 // z4_rhs_movpunc_N (spec z4_rhs_movpunc_N.m:216-397).  The order of work is

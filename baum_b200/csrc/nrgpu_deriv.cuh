@@ -1,5 +1,5 @@
 // nrgpu_deriv.cuh -- the interior right-hand side in two kernels per part of
-// a box (included inside the anonymous namespace of nrgpu_bssn.cu):
+// a box (included by nrgpu_parts.cuh):
 //
 //   deriv_kernel    per field: the stencils that several points or several
 //                   operators share.  A thread owns one (x, y) column of a
@@ -7,10 +7,10 @@
 //                   k - R .. k + R in registers.  It writes, per point, the
 //                   field's advection plus dissipation (weighted, ready to
 //                   add to its rhs) and, for the fields that need them, the
-//                   numerators d_y f, d_z f, d_zz f and d_z d_y f (from the
-//                   d_y of the planes it has passed).
-//   algebra_kernel  per point: d_x f, d_xx f, d_yy f from the field, d_x d_y f
-//                   and d_x d_z f from the stored numerators (the stencil of
+//                   numerators d_y f, d_z f and d_zz f.
+//   algebra_kernel  per point: d_x f, d_xx f, d_yy f from the field, d_x d_y f,
+//                   d_x d_z f and d_y d_z f from the stored numerators of the
+//                   columns and rows around (the stencil of
 //                   a mixed derivative is the product of two first-derivative
 //                   stencils, discretize.m:68-71), then the algebra and the
 //                   Runge-Kutta update.
@@ -19,22 +19,23 @@
 // ~1400 stencil taps per point (a 6th-order one ~2500), most of them for the
 // mixed derivatives (16 or 36 each) and for taps that several operators
 // share, and it needs every register of the SM for 8 warps that wait for
-// those taps.  Here a point costs ~330 loads and ~75 stores in the first
-// kernel and ~300 loads in the second, and neither needs compile-time box
+// those taps.  Here a point costs ~330 loads and ~70 stores in the first
+// kernel and ~350 loads in the second, and neither needs compile-time box
 // sizes.  The stored numerators lie row by row, all lists of a row side by
 // side at a fixed pitch, so that every access to them is one pointer plus a
 // constant: with a list per array the address arithmetic was two thirds of
 // the instructions that are not FP64.
 //
 // A part is at most kPartX interior points wide; only d_y f and d_z f are
-// needed beyond it (H columns on either side, which the first kernel computes
-// for both parts).  Along y and z a part has no halo.
+// needed beyond it, along x, and d_z f along y (H columns and rows on either
+// side, which the first kernel computes for both parts).  Along z a part has
+// no halo.
 
 // ---- what is stored per row of a part: lists at pitch kPitch ------------------------
 //   [0, NV)        advection + dissipation
 //   [NV, NV + 3)   advection of Gamma~ alone (only where the B equation takes it)
 //   then for the 11 fields with all second derivatives (g~, chi, alpha, beta)
-//   d_y, d_z, d_zz, d_yz, and for the others with first derivatives (Gamma~,
+//   d_y, d_z, d_zz, and for the others with first derivatives (Gamma~,
 //   K, Theta) d_y, d_z
 constexpr int kNM = 11, kPitch = 128, kColumn0 = 4, kPartX = 120;
 template <int NV>
