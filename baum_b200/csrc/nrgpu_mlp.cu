@@ -6,8 +6,9 @@
 // Network: 32 input features -> 4 hidden layers of 128 (SiLU) -> 1 output.
 // Every hidden-layer product runs on the tensor cores as BF16 x BF16 with
 // FP32 accumulation (mma.sync m16n8k16); the master weights, the Adam state,
-// biases, the output layer and the loss are FP32.  Training is the plain
-// reverse-mode chain with the same BF16 operands as the forward pass.
+// biases and the output layer are FP32, the loss is summed in 64 bits (its error
+// against a 64-bit network, 2e-5 to 4e-4 after 16 steps, is the BF16 products').
+// Training is the plain reverse-mode chain with the same BF16 operands as the forward pass.
 //
 // Kernels:
 //   mlp_features_kernel     feature rows (double math, rounded to BF16)
@@ -129,7 +130,8 @@ struct RowsArgs {
   float *out;                   // network output per row
   float *Z[4];                  // silu'(z) (training)
   __nv_bfloat16 *A[4], *dZ[4];  // activations, pre-activation gradients (training)
-  float *grad, *loss;
+  float *grad;
+  double *loss;
   int n;
 };
 
@@ -154,14 +156,17 @@ template <bool TRAIN>
 __global__ void __launch_bounds__(kRowsThreads) mlp_rows_kernel(const RowsArgs a) {
   extern __shared__ __align__(16) __nv_bfloat16 wsm[];
   __nv_bfloat16 *xsm = wsm + kWRows * kWPitch;  // two buffers of 128 rows, the operands between layers
-  __shared__ float sums[5 * HID + 2];  // db of the four layers, dw5, db5, loss
+  __shared__ float sums[5 * HID + 1];  // db of the four layers, dw5, db5
+  __shared__ double squares[kRowsThreads / 64];  // loss of each pair of warps, in 64 bits
   __shared__ float outs[2][128];       // the two halves of the output sums
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31, g = lane >> 2, tg = lane & 3;
   const int pair = warp >> 1, c0 = (warp & 1) * (HID / 2);  // 16 rows, 64 columns
   for (int q = t; q < kWRows * HID / 8; q += kRowsThreads)
     cp16(wsm + (q / (HID / 8)) * kWPitch + (q % (HID / 8)) * 8, a.Wb + (long)q * 8);
-  if (TRAIN)
-    for (int q = t; q < 5 * HID + 2; q += kRowsThreads) sums[q] = 0.0f;
+  if (TRAIN) {
+    for (int q = t; q < 5 * HID + 1; q += kRowsThreads) sums[q] = 0.0f;
+    if (t < kRowsThreads / 64) squares[t] = 0.0;
+  }
   asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
   __syncthreads();
   const int r0 = blockIdx.x * 128 + pair * 16;
@@ -263,7 +268,12 @@ __global__ void __launch_bounds__(kRowsThreads) mlp_rows_kernel(const RowsArgs a
       const float da = 2.0f * ea / (float)a.n, db = 2.0f * eb / (float)a.n;
       if (tg == 0 && c0 == 0) {
         atomicAdd(sums + 5 * HID, da + db);
-        atomicAdd(sums + 5 * HID + 1, ea * ea + eb * eb);
+      }
+      if (c0 == 0) {
+        double q = (double)ea * ea + (double)eb * eb;
+#pragma unroll
+        for (int o = 4; o < 32; o <<= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+        if (lane == 0) squares[pair] = q;
       }
 #pragma unroll
       for (int l = 3; l >= 0; --l) {
@@ -318,7 +328,9 @@ __global__ void __launch_bounds__(kRowsThreads) mlp_rows_kernel(const RowsArgs a
       atomicAdd(a.grad + (q < 4 * HID ? off_b(q / HID) + q % HID : kOffW5 + q % HID), sums[q]);
     if (t == 0) {
       atomicAdd(a.grad + kOffW5 + HID, sums[5 * HID]);
-      atomicAdd(a.loss, sums[5 * HID + 1] / (float)a.n);
+      double q = 0.0;
+      for (int w = 0; w < kRowsThreads / 64; ++w) q += squares[w];
+      atomicAdd(a.loss, q / a.n);
     }
   }
 }
@@ -849,7 +861,8 @@ struct nrgpu_mlp {
   float *Z[4];             // [max_batch][HID] silu' of the pre-activations (1 to 3)
   __nv_bfloat16 *Ab[4];    // [max_batch][HID] activations (1 to 3)
   __nv_bfloat16 *dZ[4];    // [max_batch][HID] pre-activation gradients
-  float *out, *loss;       // loss: right after G
+  float *out;
+  double *loss;            // right after G, on the next 8 bytes
   double *cond;            // the conditioning table
   int ncond;
   int *d_tcstatus;         // a wait of the tensor-core forward ran out
@@ -905,7 +918,7 @@ extern "C" int nrgpu_mlp_create(int max_batch, nrgpu_mlp **out) {
   M->max_batch = max_batch;
   const size_t nh = (size_t)max_batch * HID;
   bool ok = cudaMalloc(&M->P, sizeof(float) * kNParams) == cudaSuccess &&
-            cudaMalloc(&M->G, sizeof(float) * (kNParams + 1)) == cudaSuccess &&
+            cudaMalloc(&M->G, sizeof(float) * (kNParams + 3)) == cudaSuccess &&
             cudaMalloc(&M->Mo, sizeof(float) * kNParams) == cudaSuccess &&
             cudaMalloc(&M->Vo, sizeof(float) * kNParams) == cudaSuccess &&
             cudaMalloc(&M->Wb, sizeof(__nv_bfloat16) * (IN * HID + 3 * HID * HID)) == cudaSuccess &&
@@ -917,10 +930,10 @@ extern "C" int nrgpu_mlp_create(int max_batch, nrgpu_mlp **out) {
     ok = (l == 3 || cudaMalloc(&M->Z[l], sizeof(float) * nh) == cudaSuccess) &&
          (l == 3 || cudaMalloc(&M->Ab[l], sizeof(__nv_bfloat16) * nh) == cudaSuccess) &&
          cudaMalloc(&M->dZ[l], sizeof(__nv_bfloat16) * nh) == cudaSuccess;
-  M->loss = M->G + kNParams;
+  M->loss = (double *)(M->G + (kNParams + 1) / 2 * 2);
   if (ok)
     ok = cudaMemset(M->P, 0, sizeof(float) * kNParams) == cudaSuccess &&
-         cudaMemset(M->G, 0, sizeof(float) * (kNParams + 1)) == cudaSuccess &&
+         cudaMemset(M->G, 0, sizeof(float) * (kNParams + 3)) == cudaSuccess &&
          cudaMemset(M->Mo, 0, sizeof(float) * kNParams) == cudaSuccess &&
          cudaMemset(M->Vo, 0, sizeof(float) * kNParams) == cudaSuccess;
   if (!ok) {
@@ -991,7 +1004,7 @@ extern "C" int nrgpu_mlp_train_step(nrgpu_mlp *M, const float *d_y, int n, float
   if (!M || !d_y || n < 64 || n % 64 || n > M->max_batch)
     return nrgpu_set_error(NRGPU_ERR_ARG, "batch %d: a multiple of 64 up to %d", n, M ? M->max_batch : 0);
   const cudaStream_t st = (cudaStream_t)stream;
-  NRGPU_CUDA_TRY(cudaMemsetAsync(M->G, 0, sizeof(float) * (kNParams + 1), st));  // the gradients and the loss
+  NRGPU_CUDA_TRY(cudaMemsetAsync(M->G, 0, sizeof(float) * (kNParams + 3), st));  // the gradients and the loss
   NRGPU_CUDA_TRY(cudaFuncSetAttribute(mlp_rows_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowsSmem));
   NRGPU_CUDA_TRY(cudaFuncSetAttribute(mlp_weight_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGradSmem));
   const RowsArgs a = rows_args(M, n, d_y, M->out);
@@ -1011,8 +1024,10 @@ extern "C" int nrgpu_mlp_train_step(nrgpu_mlp *M, const float *d_y, int n, float
     NRGPU_CUDA_TRY(cudaGetLastError());
   }
   if (loss) {
-    NRGPU_CUDA_TRY(cudaMemcpyAsync(loss, M->loss, sizeof(float), cudaMemcpyDeviceToHost, st));
+    double l;
+    NRGPU_CUDA_TRY(cudaMemcpyAsync(&l, M->loss, sizeof l, cudaMemcpyDeviceToHost, st));
     NRGPU_CUDA_TRY(cudaStreamSynchronize(st));
+    *loss = (float)l;
   }
   return NRGPU_OK;
 }
