@@ -37,10 +37,10 @@ RHS_PER_STEP = 4
 # algorithmic FP64 work of one inner point: operators of the reference's
 # generated rhs (bssn_rhs_movpunc_N.c) on its 4th-order + KO6 path
 FLOP_PER_POINT = 4973
-# DRAM bytes of one RK-stage launch of bssn_rhs_kernel on the 64^3 box, block 32 x 8 x 1
-# (dram__bytes_read.sum + dram__bytes_write.sum of one ncu capture, mean of
-# the two captured launches, stages 1 and 2: 108.6 MB and 216.5 MB)
-RHS_TRAFFIC_BYTES = 162.6e6
+# DRAM bytes of the interior rhs of one RK stage on the 64^3 box
+# (dram__bytes_read.sum + dram__bytes_write.sum of one ncu capture, mean of the
+# four stages of a step: deriv_kernel 167 MB, algebra_kernel 338 MB)
+RHS_TRAFFIC_BYTES = 505e6
 CONFIG = {"workload": "bssn_schwarzschild_64^3_rk4", "box": "66^3 (64^3 inner + boundary layer)",
           "dx": DX, "dt": DT, "order": 4, "dissipation": "KO6 eps=0.1", "gauge": "1+log, Gamma-driver eta=2",
           "l2": "flushed (256 MiB write) before every timed step", "parallelism": "replicas"}
