@@ -913,34 +913,52 @@ static int launch_bssn_tile(nrgpu_level *L, int b, const CUtensorMap *maps, cons
   return NRGPU_OK;
 }
 
-// The lists belong to the level: launches on them from several host
-// threads, or on several streams, take turns (the lock, and an event of the
-// last use; a stream that is being captured is ordered by its graph).
-struct ListTurn {
+// The workspace of one interior rhs.  An RK step takes the step's.  Rhs calls
+// on several host threads or streams take turns on the call's: the lock, and
+// an event of its last use.  A captured call would leave both behind, since
+// nothing orders its replays with other graphs' or with eager calls: it gets
+// none, and runs kernels that share nothing (point by point, at run-time
+// strides where a box of its size would be staged).  Under capture nothing is
+// allocated: a captured step uses what the level's earlier steps allocated.
+struct RhsTurn {
   nrgpu_level *L;
   cudaStream_t st;
-  bool capturing;
-  ListTurn(nrgpu_level *L_, cudaStream_t st_) : L(L_), st(st_) {
+  RhsWork none, *w;
+  bool step, capturing;
+  RhsTurn(nrgpu_level *L_, cudaStream_t st_, bool step_) : L(L_), st(st_), none(), w(&none), step(step_) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     capturing = cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone;
-    // the lists are allocated here unless a graph is being captured (the
-    // refinement driver's first coarse step runs without one)
-    if (!capturing && L->parts) nrgpu_level_lists(L);
-    L->list_lock->lock();
-    if (L->lists && !capturing) cudaStreamWaitEvent(st, L->ev_lists, 0);
+    if (capturing) cudaGetLastError();
+    if (step) {
+      w = &L->step_work;
+    } else if (!capturing) {
+      L->call_lock->lock();
+      if (L->ev_call || cudaEventCreateWithFlags(&L->ev_call, cudaEventDisableTiming) == cudaSuccess) w = &L->call_work;
+      else cudaGetLastError();
+      if (shared() && cudaStreamWaitEvent(st, L->ev_call, 0) != cudaSuccess) cudaDeviceSynchronize();
+    }
+    if (may_allocate() && L->parts) nrgpu_level_lists(L, w);
   }
-  ~ListTurn() {
-    if (L->lists && !capturing) cudaEventRecord(L->ev_lists, st);
-    L->list_lock->unlock();
+  ~RhsTurn() {
+    if (step || capturing) return;
+    if (shared() && cudaEventRecord(L->ev_call, st) != cudaSuccess) cudaStreamSynchronize(st);
+    L->call_lock->unlock();
   }
-  ListTurn(const ListTurn &) = delete;
+  bool may_allocate() const { return !capturing && w != &none; }
+  bool shared() const { return w->lists || w->pad || L->queue; }  // (the queue's counter)
+  // the staging buffer, when a box runs point by point
+  void pad() {
+    if (may_allocate()) nrgpu_level_pad(L, w);
+  }
+  RhsTurn(const RhsTurn &) = delete;
 };
 
 // launch the interior and flagged kernels of one rhs evaluation
-// (kb <= k <= ke: the planes of the interior launch, whole boxes by default)
-static int launch_rhs(nrgpu_level *L, const CVarPtrs &U, const VarPtrs &out, const CVarPtrs &pre, const VarPtrs &acc,
-                      const Epilogue &E, const nrgpu_bssn_params &p, cudaStream_t st, bool interior, bool flagged,
-                      int kb = 1, int ke = 1 << 30) {
+// (step: of an RK step, see RhsTurn; kb <= k <= ke: the planes of the
+// interior launch, whole boxes by default)
+static int launch_rhs(nrgpu_level *L, bool step, const CVarPtrs &U, const VarPtrs &out, const CVarPtrs &pre,
+                      const VarPtrs &acc, const Epilogue &E, const nrgpu_bssn_params &p, cudaStream_t st, bool interior,
+                      bool flagged, int kb = 1, int ke = 1 << 30) {
   // with both parts, the boundary kernel runs on the level's side stream,
   // launched after the interior kernel so that its blocks fill the
   // interior kernel's last wave; they write disjoint points
@@ -952,15 +970,16 @@ static int launch_rhs(nrgpu_level *L, const CVarPtrs &U, const VarPtrs &out, con
     NRGPU_CUDA_TRY(cudaStreamWaitEvent(L->side, L->ev_fork, 0));
   }
   if (interior) {
-    ListTurn turn(L, st);
+    RhsTurn turn(L, st, step);
+    const RhsWork &w = *turn.w;
     for (int b = 0; b < L->nboxes; ++b) {
       const BoxGeo &bx = L->hbox[b];
       if (bx.m < 3 || bx.n < 3 || bx.o < 3) continue;
       const int k0 = max(kb, 1), k1 = min(ke, bx.o - 2);
       if (k1 < k0) continue;
       if (L->parts && !L->tile) {
-        if (p.order_centered == 4 && nrgpu_bssn_parts_o4(L, b, U.p, out.p, pre.p, acc.p, E, p, st, k0, k1)) continue;
-        if (p.order_centered == 6 && nrgpu_bssn_parts_o6(L, b, U.p, out.p, pre.p, acc.p, E, p, st, k0, k1)) continue;
+        if (p.order_centered == 4 && nrgpu_bssn_parts_o4(L, w, b, U.p, out.p, pre.p, acc.p, E, p, st, k0, k1)) continue;
+        if (p.order_centered == 6 && nrgpu_bssn_parts_o6(L, w, b, U.p, out.p, pre.p, acc.p, E, p, st, k0, k1)) continue;
       }
       if (L->tile && tile_eligible(L, b, U.p, NRGPU_NV, p.order_centered, p.advection_lopsided,
                                    p.advection_lopsided6)) {
@@ -970,9 +989,7 @@ static int launch_rhs(nrgpu_level *L, const CVarPtrs &U, const VarPtrs &out, con
         if ((e = launch_bssn_tile(L, b, maps, U, out, pre, acc, E, p, st, k0, k1))) return e;
         continue;
       }
-      // point by point; the staging buffer of off-size boxes is allocated as
-      // the lists are
-      if (!turn.capturing) nrgpu_level_pad(L);
+      turn.pad();  // point by point
       // the block shape of the level (32 x 4 x 1, or what nrgpu_level_autotune
       // measured fastest for this box); 128 or 256 threads, one point each
       const dim3 blk(L->blk[0], L->blk[1], L->blk[2]);
@@ -987,18 +1004,18 @@ static int launch_rhs(nrgpu_level *L, const CVarPtrs &U, const VarPtrs &out, con
       int3 in = make_int3(bx.noffset, bx.m, bx.n);
       int P = ord >= 4 && bx.m == bx.n ? bx.m : 0;
       const int Q = ord >= 4 ? nrgpu_pad_size(bx.m, bx.n) : 0;
-      if (Q && L->pad) {
+      if (Q && w.pad) {
         const long fs = (long)Q * Q * bx.o;
         P = 0;
-        if ((size_t)(NRGPU_NV * fs) <= L->pad_doubles) {
+        if ((size_t)(NRGPU_NV * fs) <= w.pad_doubles) {
           // the planes the launch's stencils reach (a launch on some planes:
           // the host-buffer step's slabs)
           const int H = max(max(p.order_advection, p.order_centered / 2 + 1), p.order_dissipation / 2 + 1);
           const int klo = max(0, k0 - H), khi = min(bx.o - 1, k1 + H);
           const long nb = (long)bx.m * bx.n * (khi - klo + 1);
-          pad_copy_kernel<<<dim3((unsigned)((nb + 255) / 256), NRGPU_NV), 256, 0, st>>>(U, L->pad, bx, Q, fs, klo,
+          pad_copy_kernel<<<dim3((unsigned)((nb + 255) / 256), NRGPU_NV), 256, 0, st>>>(U, w.pad, bx, Q, fs, klo,
                                                                                         khi);
-          for (int v = 0; v < NRGPU_NV; ++v) In.p[v] = L->pad + v * fs;
+          for (int v = 0; v < NRGPU_NV; ++v) In.p[v] = w.pad + v * fs;
           in = make_int3(0, Q, Q);
           P = Q;
         }
@@ -1057,7 +1074,7 @@ extern "C" int nrgpu_bssn_rhs(nrgpu_level *L, double *const *unew, double *const
     pr = cu;
   }
   Epilogue E = {c != 0.0 ? EPI_ADDLINEAR : EPI_RHS, c, 0.0, 0.0, 0};
-  return launch_rhs(L, cptrs(cu), n, cptrs(pr), n, E, *p, (cudaStream_t)stream, true, false);
+  return launch_rhs(L, false, cptrs(cu), n, cptrs(pr), n, E, *p, (cudaStream_t)stream, true, false);
 }
 
 extern "C" int nrgpu_bssn_boundary(nrgpu_level *L, double *const *unew, double *const *upre, double c,
@@ -1073,7 +1090,7 @@ extern "C" int nrgpu_bssn_boundary(nrgpu_level *L, double *const *unew, double *
     pr = cu;
   }
   Epilogue E = {c != 0.0 ? EPI_ADDLINEAR : EPI_RHS, c, 0.0, 0.0, 0};
-  if ((e = launch_rhs(L, cptrs(cu), n, cptrs(pr), n, E, *p, (cudaStream_t)stream, false, true))) return e;
+  if ((e = launch_rhs(L, false, cptrs(cu), n, cptrs(pr), n, E, *p, (cudaStream_t)stream, false, true))) return e;
   return nrgpu_level_symmetry(L, unew, NRGPU_SYSTEM_BSSN, (cudaStream_t)stream);
 }
 
@@ -1150,10 +1167,10 @@ static int rk_stage_parts(nrgpu_level *L, const RkLists &R, int sg, double dt, c
   const CVarPtrs cU = cptrs(R.U);
   const Epilogue E = stage_epilogue(sg, dt);
   switch (sg) {
-    case 0: return launch_rhs(L, cU, R.V1, cU, R.A, E, p, st, interior, flagged, kb, ke);
-    case 1: return launch_rhs(L, cptrs(R.V1), R.V2, cU, R.A, E, p, st, interior, flagged, kb, ke);
-    case 2: return launch_rhs(L, cptrs(R.V2), R.V1, cU, R.A, E, p, st, interior, flagged, kb, ke);
-    default: return launch_rhs(L, cptrs(R.V1), R.U, cU, R.A, E, p, st, interior, flagged, kb, ke);
+    case 0: return launch_rhs(L, true, cU, R.V1, cU, R.A, E, p, st, interior, flagged, kb, ke);
+    case 1: return launch_rhs(L, true, cptrs(R.V1), R.V2, cU, R.A, E, p, st, interior, flagged, kb, ke);
+    case 2: return launch_rhs(L, true, cptrs(R.V2), R.V1, cU, R.A, E, p, st, interior, flagged, kb, ke);
+    default: return launch_rhs(L, true, cptrs(R.V1), R.U, cU, R.A, E, p, st, interior, flagged, kb, ke);
   }
 }
 
@@ -1176,7 +1193,7 @@ static int rk_stage(nrgpu_level *L, const RkLists &R, int sg, double dt, const n
   VarPtrs Rp;
   for (int v = 0; v < NRGPU_NV; ++v) Rp.p[v] = RS.p[v];
   const Epilogue Er = {EPI_RHS, 0.0, 0.0, 0.0, 0, 0};
-  if ((e = launch_rhs(L, cptrs(in), Rp, cptrs(in), Rp, Er, p, st, true, true))) return e;
+  if ((e = launch_rhs(L, true, cptrs(in), Rp, cptrs(in), Rp, Er, p, st, true, true))) return e;
   if ((e = nrgpu_level_symmetry(L, Rp.p, NRGPU_SYSTEM_BSSN, st))) return e;
   const long n = (long)NRGPU_NV * L->npoints;
   rk_update_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(RS, sym_vars(out.p, NRGPU_NV),
@@ -1576,8 +1593,8 @@ static ZCVarPtrs z4_c(const ZVarPtrs &v) {
 // Generic strides remain for larger boxes; one kernel per stencil order.
 template <int ORD>
 static void z4_interior_fp64(const ZCVarPtrs &U, const ZVarPtrs &out, const ZCVarPtrs &pre, const ZVarPtrs &acc,
-                             const Epilogue &E, const nrgpu_z4_params &p, const BoxGeo &bx, nrgpu_level *L, dim3 grd,
-                             dim3 blk, cudaStream_t st) {
+                             const Epilogue &E, const nrgpu_z4_params &p, const BoxGeo &bx, nrgpu_level *L,
+                             const RhsWork &w, dim3 grd, dim3 blk, cudaStream_t st) {
 #define NRGPU_Z4_FIXED(M_)                                                                                   \
   if (P == M_) {                                                                                             \
     z4_rhs_kernel<M_, M_ * M_, 0, ORD><<<grd, blk, 0, st>>>(In, out, pre, acc, E, p, bx, L->d_boundary, L->dx, \
@@ -1589,14 +1606,14 @@ static void z4_interior_fp64(const ZCVarPtrs &U, const ZVarPtrs &out, const ZCVa
     int3 in = make_int3(bx.noffset, bx.m, bx.n);
     int P = bx.m == bx.n ? bx.m : 0;  // a kernel of its own, if one below matches
     const int Q = nrgpu_pad_size(bx.m, bx.n);
-    if (Q && L->pad) {
+    if (Q && w.pad) {
       P = Q;
       const long fs = (long)P * P * bx.o;
-      if ((size_t)(NRGPU_Z4_NVARS * fs) <= L->pad_doubles) {
+      if ((size_t)(NRGPU_Z4_NVARS * fs) <= w.pad_doubles) {
         const long nb = (long)bx.m * bx.n * bx.o;
-        pad_copy_kernel<<<dim3((unsigned)((nb + 255) / 256), NRGPU_Z4_NVARS), 256, 0, st>>>(U, L->pad, bx, P, fs, 0,
+        pad_copy_kernel<<<dim3((unsigned)((nb + 255) / 256), NRGPU_Z4_NVARS), 256, 0, st>>>(U, w.pad, bx, P, fs, 0,
                                                                                               bx.o - 1);
-        for (int v = 0; v < NRGPU_Z4_NVARS; ++v) In.p[v] = L->pad + v * fs;
+        for (int v = 0; v < NRGPU_Z4_NVARS; ++v) In.p[v] = w.pad + v * fs;
         in = make_int3(0, P, P);
       } else {
         P = 0;
@@ -1641,8 +1658,9 @@ static int z4_queue_size(const nrgpu_level *L, const nrgpu_z4_params &p) {
 }
 
 // the interior of all boxes of the level by z4_rhs_queue_kernel
-static int z4_queue_launch(nrgpu_level *L, int m, const ZCVarPtrs &U, const ZVarPtrs &out, const ZCVarPtrs &pre,
-                           const ZVarPtrs &acc, const Epilogue &E, const nrgpu_z4_params &p, cudaStream_t st) {
+static int z4_queue_launch(nrgpu_level *L, int m, int *counter, const ZCVarPtrs &U, const ZVarPtrs &out,
+                           const ZCVarPtrs &pre, const ZVarPtrs &acc, const Epilogue &E, const nrgpu_z4_params &p,
+                           cudaStream_t st) {
   const BoxGeo &b0 = L->hbox[0];
   const dim3 blk(L->blk[0], L->blk[1], L->blk[2]);
   const int3 tiles = make_int3((b0.m - 2 + blk.x - 1) / blk.x, (b0.n - 2 + blk.y - 1) / blk.y,
@@ -1651,7 +1669,6 @@ static int z4_queue_launch(nrgpu_level *L, int m, const ZCVarPtrs &U, const ZVar
   // resident blocks: one or two per SM at 255 registers; more would wait
   const int per_sm = blk.x * blk.y * blk.z <= 128 ? 2 : 1;
   const int grid = min(total, L->nsm * per_sm);
-  int *counter = L->d_status + 2;
   NRGPU_CUDA_TRY(cudaMemsetAsync(counter, 0, sizeof(int), st));
 #define NR_Z4Q(M_, O_)                                                                                               \
   z4_rhs_queue_kernel<M_, M_ * M_, O_><<<grid, blk, 0, st>>>(U, out, pre, acc, E, p, L->d_box, L->nboxes, tiles,       \
@@ -1669,7 +1686,7 @@ static int z4_queue_launch(nrgpu_level *L, int m, const ZCVarPtrs &U, const ZVar
   return NRGPU_OK;
 }
 
-static int z4_launch(nrgpu_level *L, const ZCVarPtrs &U, const ZVarPtrs &out, const ZCVarPtrs &pre,
+static int z4_launch(nrgpu_level *L, bool step, const ZCVarPtrs &U, const ZVarPtrs &out, const ZCVarPtrs &pre,
                      const ZVarPtrs &acc, const Epilogue &E, const nrgpu_z4_params &p, cudaStream_t st, bool interior,
                      bool flagged) {
   // the boundary kernel beside the interior kernel, as in launch_rhs
@@ -1681,11 +1698,12 @@ static int z4_launch(nrgpu_level *L, const ZCVarPtrs &U, const ZVarPtrs &out, co
     NRGPU_CUDA_TRY(cudaStreamWaitEvent(L->side, L->ev_fork, 0));
   }
   if (interior) {
-    ListTurn turn(L, st);
+    RhsTurn turn(L, st, step);
+    const RhsWork &w = *turn.w;
     // all boxes in one persistent launch (nrgpu_level_queue), or one launch per box
-    const int qm = L->queue && !L->parts ? z4_queue_size(L, p) : 0;
+    const int qm = L->queue && !L->parts && (step || !turn.capturing) ? z4_queue_size(L, p) : 0;
     if (qm) {
-      int e = z4_queue_launch(L, qm, U, out, pre, acc, E, p, st);
+      int e = z4_queue_launch(L, qm, L->d_status + (step ? 2 : 3), U, out, pre, acc, E, p, st);
       if (e) return e;
     }
     for (int b = 0; b < L->nboxes && !qm; ++b) {
@@ -1693,19 +1711,19 @@ static int z4_launch(nrgpu_level *L, const ZCVarPtrs &U, const ZVarPtrs &out, co
       if (bx.m < 3 || bx.n < 3 || bx.o < 3) continue;
       if (L->parts && p.precision == 0) {
         const int k1 = bx.o - 2;
-        if (p.order_centered == 4 && nrgpu_z4_parts_o4(L, b, U.p, out.p, pre.p, acc.p, E, p, st, 1, k1)) continue;
-        if (p.order_centered == 6 && nrgpu_z4_parts_o6(L, b, U.p, out.p, pre.p, acc.p, E, p, st, 1, k1)) continue;
+        if (p.order_centered == 4 && nrgpu_z4_parts_o4(L, w, b, U.p, out.p, pre.p, acc.p, E, p, st, 1, k1)) continue;
+        if (p.order_centered == 6 && nrgpu_z4_parts_o6(L, w, b, U.p, out.p, pre.p, acc.p, E, p, st, 1, k1)) continue;
       }
-      if (!turn.capturing) nrgpu_level_pad(L);
+      turn.pad();
       // the block shape of the level (32 x 4 x 1, or what nrgpu_level_autotune
       // measured fastest for this box); 128 or 256 threads, one point each
       const dim3 blk(L->blk[0], L->blk[1], L->blk[2]);
       const dim3 grd((bx.m - 2 + blk.x - 1) / blk.x, (bx.n - 2 + blk.y - 1) / blk.y, (bx.o - 2 + blk.z - 1) / blk.z);
       if (p.precision == 1) z4_interior_prec<1>(U, out, pre, acc, E, p, bx, L, grd, blk, st);
       else if (p.precision == 2) z4_interior_prec<2>(U, out, pre, acc, E, p, bx, L, grd, blk, st);
-      else if (p.order_centered == 2) z4_interior_fp64<2>(U, out, pre, acc, E, p, bx, L, grd, blk, st);
-      else if (p.order_centered == 4) z4_interior_fp64<4>(U, out, pre, acc, E, p, bx, L, grd, blk, st);
-      else z4_interior_fp64<6>(U, out, pre, acc, E, p, bx, L, grd, blk, st);
+      else if (p.order_centered == 2) z4_interior_fp64<2>(U, out, pre, acc, E, p, bx, L, w, grd, blk, st);
+      else if (p.order_centered == 4) z4_interior_fp64<4>(U, out, pre, acc, E, p, bx, L, w, grd, blk, st);
+      else z4_interior_fp64<6>(U, out, pre, acc, E, p, bx, L, w, grd, blk, st);
     }
     // the ladder points of all boxes (beside the interior kernel)
     const int nlad = L->nladder[p.order_centered / 2 - 1];
@@ -1734,8 +1752,8 @@ static int z4_launch(nrgpu_level *L, const ZCVarPtrs &U, const ZVarPtrs &out, co
   return NRGPU_OK;
 }
 
-extern "C" int nrgpu_z4_rhs(nrgpu_level *L, double *const *unew, double *const *upre, double c, double *const *ucur,
-                            const nrgpu_z4_params *p, void *stream) {
+int nrgpu_z4_rhs_of(nrgpu_level *L, bool step, double *const *unew, double *const *upre, double c,
+                    double *const *ucur, const nrgpu_z4_params *p, cudaStream_t st) {
   if (!L) return nrgpu_set_error(NRGPU_ERR_ARG, "null level");
   int e;
   if ((e = z4_check_params(p))) return e;
@@ -1747,9 +1765,14 @@ extern "C" int nrgpu_z4_rhs(nrgpu_level *L, double *const *unew, double *const *
     pr = cu;
   }
   // the background boundary extrapolates the state onto the boundary first
-  if (p->boundary && (e = nrgpu_z4_background_extrapolate(L, ucur, (cudaStream_t)stream))) return e;
+  if (p->boundary && (e = nrgpu_z4_background_extrapolate(L, ucur, st))) return e;
   Epilogue E = {c != 0.0 ? EPI_ADDLINEAR : EPI_RHS, c, 0.0, 0.0, 0};
-  return z4_launch(L, z4_c(cu), n, z4_c(pr), n, E, *p, (cudaStream_t)stream, true, false);
+  return z4_launch(L, step, z4_c(cu), n, z4_c(pr), n, E, *p, st, true, false);
+}
+
+extern "C" int nrgpu_z4_rhs(nrgpu_level *L, double *const *unew, double *const *upre, double c, double *const *ucur,
+                            const nrgpu_z4_params *p, void *stream) {
+  return nrgpu_z4_rhs_of(L, false, unew, upre, c, ucur, p, (cudaStream_t)stream);
 }
 
 extern "C" int nrgpu_z4_boundary(nrgpu_level *L, double *const *unew, double *const *upre, double c,
@@ -1765,7 +1788,7 @@ extern "C" int nrgpu_z4_boundary(nrgpu_level *L, double *const *unew, double *co
   }
   if (p->boundary) return nrgpu_z4_background_boundary(L, unew, upre, c, ucur, p, (cudaStream_t)stream);
   Epilogue E = {c != 0.0 ? EPI_ADDLINEAR : EPI_RHS, c, 0.0, 0.0, 0};
-  if ((e = z4_launch(L, z4_c(cu), n, z4_c(pr), n, E, *p, (cudaStream_t)stream, false, true))) return e;
+  if ((e = z4_launch(L, false, z4_c(cu), n, z4_c(pr), n, E, *p, (cudaStream_t)stream, false, true))) return e;
   return nrgpu_level_symmetry(L, unew, NRGPU_SYSTEM_Z4C, (cudaStream_t)stream);
 }
 
@@ -1803,7 +1826,7 @@ int nrgpu_z4_rk4_stages(nrgpu_level *L, double *const *u, double dt, const nrgpu
     const Epilogue Er = {EPI_RHS, 0.0, 0.0, 0.0, 0, 0};
     const ZVarPtrs *ins[4] = {&U, &V1, &V2, &V1}, *outs[4] = {&V1, &V2, &V1, &U};
     for (int sg = 0; sg < 4; ++sg) {
-      if ((e = z4_launch(L, z4_c(*ins[sg]), Rp, z4_c(*ins[sg]), Rp, Er, *p, st, true, true))) return e;
+      if ((e = z4_launch(L, true, z4_c(*ins[sg]), Rp, z4_c(*ins[sg]), Rp, Er, *p, st, true, true))) return e;
       if ((e = nrgpu_level_symmetry(L, Rp.p, NRGPU_SYSTEM_Z4C, st))) return e;
       const long n = (long)ZNV * L->npoints;
       rk_update_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(RS, sym_vars(outs[sg]->p, ZNV), sym_vars(U.p, ZNV),
@@ -1813,10 +1836,10 @@ int nrgpu_z4_rk4_stages(nrgpu_level *L, double *const *u, double dt, const nrgpu
     }
     return NRGPU_OK;
   }
-  if ((e = z4_launch(L, cU, V1, cU, A, E1, *p, st, true, true))) return e;
-  if ((e = z4_launch(L, z4_c(V1), V2, cU, A, E2, *p, st, true, true))) return e;
-  if ((e = z4_launch(L, z4_c(V2), V1, cU, A, E3, *p, st, true, true))) return e;
-  if ((e = z4_launch(L, z4_c(V1), U, cU, A, E4, *p, st, true, true))) return e;
+  if ((e = z4_launch(L, true, cU, V1, cU, A, E1, *p, st, true, true))) return e;
+  if ((e = z4_launch(L, true, z4_c(V1), V2, cU, A, E2, *p, st, true, true))) return e;
+  if ((e = z4_launch(L, true, z4_c(V2), V1, cU, A, E3, *p, st, true, true))) return e;
+  if ((e = z4_launch(L, true, z4_c(V1), U, cU, A, E4, *p, st, true, true))) return e;
   return NRGPU_OK;
 }
 
@@ -1892,7 +1915,7 @@ extern "C" int nrgpu_level_autotune(nrgpu_level *L, int system, const void *para
   }
   for (int b = 0; b < L->nboxes; ++b)
     parts = parts && (long)L->hbox[b].m * L->hbox[b].n * L->hbox[b].o >= 2 * NRGPU_PARTS_MIN_POINTS;
-  if (parts && L->parts && L->lists) {
+  if (parts && L->parts && L->step_work.lists) {
     L->tile = 0;
     for (int q = 0; q < 3; ++q)
       if (best_block) best_block[q] = L->blk[q];
@@ -1913,14 +1936,14 @@ extern "C" int nrgpu_level_autotune(nrgpu_level *L, int system, const void *para
           P.p[v] = scr + (long)v * np;
           O.p[v] = scr + (long)(ZNV + v) * np;
         }
-        e = launch_rhs(L, cptrs(P), O, cptrs(P), O, E, *(const nrgpu_bssn_params *)params, st, true, false);
+        e = launch_rhs(L, true, cptrs(P), O, cptrs(P), O, E, *(const nrgpu_bssn_params *)params, st, true, false);
       } else {
         ZVarPtrs P, O;
         for (int v = 0; v < ZNV; ++v) {
           P.p[v] = scr + (long)v * np;
           O.p[v] = scr + (long)(ZNV + v) * np;
         }
-        e = z4_launch(L, z4_c(P), O, z4_c(P), O, E, *(const nrgpu_z4_params *)params, st, true, false);
+        e = z4_launch(L, true, z4_c(P), O, z4_c(P), O, E, *(const nrgpu_z4_params *)params, st, true, false);
       }
     }
     cudaEventRecord(ev1, st);
@@ -1951,7 +1974,7 @@ extern "C" int nrgpu_level_autotune(nrgpu_level *L, int system, const void *para
       L->tile = mode;
       for (int rep = 0; rep < 4 && !e; ++rep) {
         if (rep == 1) cudaEventRecord(ev0, st);
-        e = launch_rhs(L, cptrs(P), O, cptrs(P), O, E, bp, st, true, false);
+        e = launch_rhs(L, true, cptrs(P), O, cptrs(P), O, E, bp, st, true, false);
       }
       cudaEventRecord(ev1, st);
       cudaEventSynchronize(ev1);
@@ -1977,7 +2000,7 @@ extern "C" int nrgpu_level_autotune(nrgpu_level *L, int system, const void *para
     L->queue = 1;
     for (int rep = 0; rep < 4 && !e; ++rep) {
       if (rep == 1) cudaEventRecord(ev0, st);
-      e = z4_launch(L, z4_c(P), O, z4_c(P), O, E, zp, st, true, false);
+      e = z4_launch(L, true, z4_c(P), O, z4_c(P), O, E, zp, st, true, false);
     }
     cudaEventRecord(ev1, st);
     cudaEventSynchronize(ev1);

@@ -37,6 +37,20 @@ struct Epilogue {
   int accmode;     // EPI_RK: ACC_ADD / ACC_INIT / ACC_FINAL
 };
 
+// what the interior rhs keeps beside the fields, allocated on first use: the
+// lists that the two kernels of nrgpu_deriv.cuh pass from one to the other
+// (rows of NRGPU_DERIV_LISTS x NRGPU_DERIV_PITCH doubles), and the staging
+// buffer of a box whose size has no compile-time-stride kernel
+// (pad_copy_kernel).  Launches that use one of these must not overlap.
+struct RhsWork {
+  double *lists;
+  size_t list_rows;
+  int lists_tried;
+  double *pad;
+  size_t pad_doubles;
+  int pad_tried;
+};
+
 struct nrgpu_level {
   int device;
   int nboxes;
@@ -52,27 +66,23 @@ struct nrgpu_level {
   FlagPoint *d_ladder;
   int nladder[3];
   BoxGeo *d_box;           // boxes on the device
-  int *d_status;           // [0]: NaN flag, [1]: inner point without stencil room
+  // [0]: NaN flag, [1]: inner point without stencil room, [2], [3]: the queue
+  // kernel's tile counters (of the RK steps, of the rhs calls)
+  int *d_status;
   // RK4 scratch: three full 24-variable lists, allocated on first use
   double *scratch;
   size_t scratch_points;
-  // staging buffer of a box whose size has no compile-time-stride kernel
-  // (pad_copy_kernel), allocated with the scratch when a box needs it
-  double *pad;
-  size_t pad_doubles;
-  int pad_tried;
   // 1: the interior rhs by the two kernels of nrgpu_deriv.cuh where they
   // cover the run; 0: point by point (the levels of a deep hierarchy,
   // nrgpu_fmr_create)
   int parts;
-  // the lists of those kernels (first use): rows of
-  // NRGPU_DERIV_LISTS x NRGPU_DERIV_PITCH doubles; the lock and the event of
-  // their last use
-  double *lists;
-  size_t list_rows;
-  int lists_tried;
-  std::mutex *list_lock;
-  cudaEvent_t ev_lists;
+  // step_work: of the RK steps, which no more overlap each other than they
+  // may on the scratch.  call_work: of the rhs calls, which otherwise share
+  // nothing and may come from several threads and streams: the lock, and the
+  // event of its last use (RhsTurn)
+  RhsWork step_work, call_work;
+  std::mutex *call_lock;
+  cudaEvent_t ev_call;
   // device copy of a host state for the host-buffer entry points
   double *hoststate;
   // points with boundary flag 0, and the norm reduction buffer (first use)
@@ -118,6 +128,9 @@ int nrgpu_z4_algcon(nrgpu_level *L, double *const *u, const nrgpu_z4_params *p, 
 int nrgpu_z4_background_extrapolate(nrgpu_level *L, double *const *u, cudaStream_t st);
 int nrgpu_z4_background_boundary(nrgpu_level *L, double *const *unew, double *const *upre, double c,
                                  double *const *ucur, const nrgpu_z4_params *p, cudaStream_t st);
+// nrgpu_z4_rhs, as a call of its own or inside an RK step
+int nrgpu_z4_rhs_of(nrgpu_level *L, bool step, double *const *unew, double *const *upre, double c,
+                    double *const *ucur, const nrgpu_z4_params *p, cudaStream_t st);
 int nrgpu_z4_rk4_background(nrgpu_level *L, double *const *u, double dt, const nrgpu_z4_params *p, cudaStream_t st);
 // the level's three RK4 scratch lists, allocated on first use (nrgpu_lib.cu)
 int nrgpu_level_scratch(nrgpu_level *L, double **out);
@@ -135,33 +148,33 @@ inline int nrgpu_pad_size(int m, int n) {
     if (c >= m && c >= n) return c;
   return 0;
 }
-void nrgpu_level_pad(nrgpu_level *L);
-// the lists of the two rhs kernels, allocated once per level; a level without
-// them runs the point-by-point kernels (nrgpu_lib.cu)
+void nrgpu_level_pad(const nrgpu_level *L, RhsWork *w);
+// the lists of the two rhs kernels, tried once per workspace; without them
+// the point-by-point kernels run (nrgpu_lib.cu)
 #define NRGPU_DERIV_LISTS 71
 #define NRGPU_DERIV_PITCH 128
 #define NRGPU_PARTS_MIN_POINTS 50000
 #define NRGPU_PARTS_MAX_LEVELS 5
-void nrgpu_level_lists(nrgpu_level *L);
+void nrgpu_level_lists(const nrgpu_level *L, RhsWork *w);
 // whether those kernels have the run's advection rows: shifts 1 and 2
 // (centred) at 4th order, 2 and 3 (centred) at 6th
 inline bool nrgpu_parts_cover(int order, int lop, int lop6) {
   return order == 4 ? lop == 1 || lop == 2 : order == 6 && (lop6 == 2 || lop6 == 3);
 }
 // interior rhs of box b on planes kb .. ke by those kernels, per system and
-// order; false when they do not apply (nrgpu_parts_*.cu)
-bool nrgpu_bssn_parts_o4(nrgpu_level *L, int b, const double *const *U, double *const *out, const double *const *pre,
-                         double *const *acc, const Epilogue &E, const nrgpu_bssn_params &p, cudaStream_t st, int kb,
-                         int ke);
-bool nrgpu_bssn_parts_o6(nrgpu_level *L, int b, const double *const *U, double *const *out, const double *const *pre,
-                         double *const *acc, const Epilogue &E, const nrgpu_bssn_params &p, cudaStream_t st, int kb,
-                         int ke);
-bool nrgpu_z4_parts_o4(nrgpu_level *L, int b, const double *const *U, double *const *out, const double *const *pre,
-                       double *const *acc, const Epilogue &E, const nrgpu_z4_params &p, cudaStream_t st, int kb,
-                       int ke);
-bool nrgpu_z4_parts_o6(nrgpu_level *L, int b, const double *const *U, double *const *out, const double *const *pre,
-                       double *const *acc, const Epilogue &E, const nrgpu_z4_params &p, cudaStream_t st, int kb,
-                       int ke);
+// order, with the lists of w; false when they do not apply (nrgpu_parts_*.cu)
+bool nrgpu_bssn_parts_o4(nrgpu_level *L, const RhsWork &w, int b, const double *const *U, double *const *out,
+                         const double *const *pre, double *const *acc, const Epilogue &E, const nrgpu_bssn_params &p,
+                         cudaStream_t st, int kb, int ke);
+bool nrgpu_bssn_parts_o6(nrgpu_level *L, const RhsWork &w, int b, const double *const *U, double *const *out,
+                         const double *const *pre, double *const *acc, const Epilogue &E, const nrgpu_bssn_params &p,
+                         cudaStream_t st, int kb, int ke);
+bool nrgpu_z4_parts_o4(nrgpu_level *L, const RhsWork &w, int b, const double *const *U, double *const *out,
+                       const double *const *pre, double *const *acc, const Epilogue &E, const nrgpu_z4_params &p,
+                       cudaStream_t st, int kb, int ke);
+bool nrgpu_z4_parts_o6(nrgpu_level *L, const RhsWork &w, int b, const double *const *U, double *const *out,
+                       const double *const *pre, double *const *acc, const Epilogue &E, const nrgpu_z4_params &p,
+                       cudaStream_t st, int kb, int ke);
 // set_boundary_symmetry on a list of nv variables of the given system
 // (NRGPU_SYSTEM_BSSN / _Z4C); nothing without symmetry (nrgpu_bssn.cu)
 int nrgpu_level_symmetry(nrgpu_level *L, double *const *u, int system, cudaStream_t st);

@@ -144,8 +144,8 @@ extern "C" int nrgpu_level_create(const nrgpu_level_desc *d, nrgpu_level **out) 
   }
   nrgpu_level *L = (nrgpu_level *)calloc(1, sizeof(nrgpu_level));
   if (!L) return nrgpu_set_error(NRGPU_ERR_NOMEM, "host allocation");
-  L->list_lock = new (std::nothrow) std::mutex;
-  if (!L->list_lock) {
+  L->call_lock = new (std::nothrow) std::mutex;
+  if (!L->call_lock) {
     free(L);
     return nrgpu_set_error(NRGPU_ERR_NOMEM, "host allocation");
   }
@@ -200,10 +200,12 @@ extern "C" int nrgpu_level_destroy(nrgpu_level *L) {
   cudaFree(L->d_sym);
   cudaFree(L->rsym);
   cudaFree(L->scratch);
-  cudaFree(L->pad);
-  cudaFree(L->lists);
-  if (L->ev_lists) cudaEventDestroy(L->ev_lists);
-  delete L->list_lock;
+  for (RhsWork *w : {&L->step_work, &L->call_work}) {
+    cudaFree(w->pad);
+    cudaFree(w->lists);
+  }
+  if (L->ev_call) cudaEventDestroy(L->ev_call);
+  delete L->call_lock;
   cudaFree(L->hoststate);
   cudaFree(L->d_red);
   cudaFree(L->d_red0d);
@@ -224,45 +226,42 @@ extern "C" int nrgpu_level_destroy(nrgpu_level *L) {
 
 // the staging buffer for boxes of up to 194 points per side without a
 // compile-time-stride kernel of their own: 25 lists with strides (1, P, P P),
-// P the next kernel size (kPadSizes); tried once per level, and a level
-// without it runs those boxes with the run-time-stride kernel
-void nrgpu_level_pad(nrgpu_level *L) {
-  if (L->pad_tried) return;
-  L->pad_tried = 1;
+// P the next kernel size (kPadSizes); tried once per workspace, and without it
+// those boxes run the run-time-stride kernel
+void nrgpu_level_pad(const nrgpu_level *L, RhsWork *w) {
+  if (w->pad_tried) return;
+  w->pad_tried = 1;
   size_t need = 0;
   for (int b = 0; b < L->nboxes; ++b) {
     const int P = nrgpu_pad_size(L->hbox[b].m, L->hbox[b].n);
     if (P > 0) need = std::max(need, (size_t)NRGPU_Z4_NVARS * P * P * L->hbox[b].o);
   }
-  if (need && cudaMalloc(&L->pad, sizeof(double) * need) == cudaSuccess) {
-    L->pad_doubles = need;
+  if (need && cudaMalloc(&w->pad, sizeof(double) * need) == cudaSuccess) {
+    w->pad_doubles = need;
   } else {
     cudaGetLastError();
-    L->pad = nullptr;
-    L->pad_doubles = 0;
+    w->pad = nullptr;
+    w->pad_doubles = 0;
   }
 }
 
 // The lists that the two rhs kernels pass from one to the other, for as many
 // rows of a part of the largest box as kListBytes hold.
 constexpr size_t kListBytes = (size_t)512 << 20;
-void nrgpu_level_lists(nrgpu_level *L) {
-  std::lock_guard<std::mutex> g(*L->list_lock);
-  if (L->lists_tried) return;
-  L->lists_tried = 1;
+void nrgpu_level_lists(const nrgpu_level *L, RhsWork *w) {
+  if (w->lists_tried) return;
+  w->lists_tried = 1;
   constexpr size_t row = sizeof(double) * NRGPU_DERIV_LISTS * NRGPU_DERIV_PITCH;
   size_t rows = 0;
   for (int b = 0; b < L->nboxes; ++b)
     if ((long)L->hbox[b].m * L->hbox[b].n * L->hbox[b].o >= NRGPU_PARTS_MIN_POINTS)
       rows = std::max(rows, (size_t)L->hbox[b].n * std::max(0, L->hbox[b].o - 4));
   rows = std::min(rows, kListBytes / row);
-  if (rows && cudaMalloc(&L->lists, rows * row) == cudaSuccess &&
-      cudaEventCreateWithFlags(&L->ev_lists, cudaEventDisableTiming) == cudaSuccess) {
-    L->list_rows = rows;
+  if (rows && cudaMalloc(&w->lists, rows * row) == cudaSuccess) {
+    w->list_rows = rows;
   } else {
     cudaGetLastError();
-    cudaFree(L->lists);
-    L->lists = nullptr;
+    w->lists = nullptr;
   }
 }
 
@@ -277,8 +276,8 @@ int nrgpu_level_scratch(nrgpu_level *L, double **out) {
       return nrgpu_set_error(NRGPU_ERR_NOMEM, "RK4 scratch of %zu bytes", bytes);
     }
     L->scratch_points = (size_t)L->npoints;
-    if (L->parts) nrgpu_level_lists(L);
-    if (!L->lists) nrgpu_level_pad(L);
+    if (L->parts) nrgpu_level_lists(L, &L->step_work);
+    if (!L->step_work.lists) nrgpu_level_pad(L, &L->step_work);
   }
   *out = L->scratch;
   return NRGPU_OK;

@@ -62,11 +62,12 @@ int part_size(int n, int most) {
 // nrgpu_deriv.cuh, part by part; false when they do not apply (nothing
 // launched then)
 template <int NV, int ORD, class PARAMS>
-bool launch_parts(nrgpu_level *L, int b, const double *const *U, double *const *out, const double *const *pre,
-                  double *const *acc, const Epilogue &E, const PARAMS &p, cudaStream_t st, int kb, int ke) {
+bool launch_parts(nrgpu_level *L, const RhsWork &w, int b, const double *const *U, double *const *out,
+                  const double *const *pre, double *const *acc, const Epilogue &E, const PARAMS &p, cudaStream_t st,
+                  int kb, int ke) {
   constexpr int H = ORD / 2;
   const int lop = ORD == 4 ? p.advection_lopsided : p.advection_lopsided6;
-  if (!nrgpu_parts_cover(ORD, p.advection_lopsided, p.advection_lopsided6) || L->list_rows <= 2 * H) return false;
+  if (!nrgpu_parts_cover(ORD, p.advection_lopsided, p.advection_lopsided6) || w.list_rows <= 2 * H) return false;
   const BoxGeo &bx = L->hbox[b];
   const int z0 = std::max(kb, H), z1 = std::min(ke, bx.o - 1 - H);
   const int nx = bx.m - 2 * H, ny = bx.n - 2 * H, nz = z1 - z0 + 1;
@@ -74,7 +75,7 @@ bool launch_parts(nrgpu_level *L, int b, const double *const *U, double *const *
   // small boxes leave most SMs idle either way, and one launch is cheaper than
   // two: 34^3 step 217 us point by point against 222, 50^3 774 against 563
   if ((long)nx * ny * (bx.o - 2 * H) < kPartsMinPoints) return false;
-  const size_t rows = L->list_rows;
+  const size_t rows = w.list_rows;
   const int px = part_size(nx, kPartX);
   const int py = part_size(ny, (int)std::min<size_t>(rows - 2 * H, ny));
   const int pz = part_size(nz, (int)std::min<size_t>(rows / (py + 2 * H), nz));
@@ -94,7 +95,7 @@ bool launch_parts(nrgpu_level *L, int b, const double *const *U, double *const *
   sa.w2 = E.cv;
   sa.has2 = E.mode == EPI_RK && !last && E.has_v;
   g.c = deriv_scale(ORD, L->dx, L->dy, L->dz);
-  g.ws = d.ws = L->lists;
+  g.ws = d.ws = w.lists;
   g.flag = L->d_boundary + bx.noffset;
   d.rst = ORD - lop;
   d.dmin = p.order_dissipation == 4 ? 2 : 3;

@@ -189,7 +189,7 @@ int nrgpu_z4_rk4_background(nrgpu_level *L, double *const *u, double dt, const n
       NRGPU_CUDA_TRY(cudaGetLastError());
       cur = pv;
     }
-    if ((e = nrgpu_z4_rhs(L, pr, pup, 0.0, cur, p, st))) return e;
+    if ((e = nrgpu_z4_rhs_of(L, true, pr, pup, 0.0, cur, p, st))) return e;
     if ((e = nrgpu_z4_background_boundary(L, pr, pup, 0.0, cur, p, st))) return e;
     axpy_kernel<<<g, 256, 0, st>>>(U, U, b[s], R, np);  // u += b r
     NRGPU_CUDA_TRY(cudaGetLastError());

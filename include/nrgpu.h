@@ -498,7 +498,13 @@ enum { NRGPU_SYSTEM_BSSN = 0, NRGPU_SYSTEM_Z4C = 1 };
  * rhs in two kernels that choose their own tiles (advection shifts 1 and 2 at
  * 4th order, 2 and 3 at 6th; FP64; not on the levels of a hierarchy deeper
  * than five): there nothing is timed and the level's shape stays.  Their
- * intermediate lists take up to 512 MB per level, allocated on first use.
+ * intermediate lists take up to 512 MB per level for the RK steps and as much
+ * again for nrgpu_bssn_rhs and nrgpu_z4_rhs, each allocated on its first use
+ * outside a graph capture.  rhs calls of one level may overlap (host threads,
+ * streams, graphs), RK steps of one level may not: they share its scratch.  A
+ * captured rhs call runs point by point, a captured RK step the kernels of an
+ * eager one with what earlier steps of the level allocated; without memory for
+ * the lists the point-by-point kernels run.  The two round differently.
  * The other rhs kernels compute one point per thread in blocks of 128 or 256
  * threads.  nrgpu_level_autotune times twenty block shapes (x, y, z
  * extents, from 32 x 4 x 1 and 8 x 16 x 1 to 8 x 4 x 4, 16 x 8 x 2 and

@@ -95,3 +95,85 @@ def test_two_streams_share_the_lists(gpu):
         for g in got:
             assert torch.equal(want, g)
     dl.close()
+
+
+def replay(graphs, streams, times):
+    for _ in range(times):
+        for g, s in zip(graphs, streams):
+            with torch.cuda.stream(s):
+                g.replay()
+
+
+def capture(stream, fn):
+    stream.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=stream):
+        fn(stream)
+    return g
+
+
+@pytest.mark.parametrize("system", ["bssn", "z4"])
+@pytest.mark.parametrize("over", [{}, {"advection_lopsided": 0}])   # two kernels; staged, point by point
+def test_captured_rhs_calls_overlap(gpu, system, over):
+    """rhs calls of one level captured into two graphs (after an eager call)
+    and replayed on two streams beside eager calls on a third: each result
+    equals the one of its own call alone, bit for bit."""
+    lev = box(60, 52, 44)
+    mod, p = (bssn, abi.bssn_params(**over)) if system == "bssn" else (z4, abi.z4_params(**over))
+    rhs = bssn.bssn_rhs_movpunc_N if system == "bssn" else z4.z4_rhs_movpunc_N
+    dl = mod.DeviceLevel(lev)
+    us = [torch.from_numpy(state(lev, system) * f).cuda() for f in (1.0, 1.001, 0.999)]
+    rs = [torch.zeros_like(u) for u in us]
+    rhs(dl, rs[2], us[2], 0.0, us[2], p)
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in us]
+    graphs = [capture(s, lambda st, u=u, r=r: rhs(dl, r, u, 0.0, u, p, st)) for u, r, s in zip(us[:2], rs, streams)]
+    for g, s in zip(graphs, streams):
+        replay([g], [s], 1)
+        torch.cuda.synchronize()
+    alone = [r.clone() for r in rs]
+    for _ in range(4):
+        for r in rs:
+            r.zero_()
+        torch.cuda.synchronize()
+        for _ in range(6):
+            replay(graphs, streams, 1)
+            rhs(dl, rs[2], us[2], 0.0, us[2], p, streams[2])
+        torch.cuda.synchronize()
+        for want, got in zip(alone, rs):
+            assert torch.equal(want, got)
+    # and they are the rhs: the eager one of the same state, up to rounding
+    r = torch.zeros_like(us[0])
+    rhs(dl, r, us[0], 0.0, us[0], p)
+    assert relerr(r.cpu().numpy(), rs[0].cpu().numpy()).max() < TOL
+    del graphs
+    dl.close()
+
+
+@pytest.mark.parametrize("system", ["bssn", "z4"])
+def test_captured_step_is_the_eager_step(gpu, system):
+    """An RK4 step replayed from a graph equals eager steps bit for bit, also
+    with an eager rhs call of the level on another stream beside it."""
+    lev = box(60, 52, 44)
+    mod, p = (bssn, abi.bssn_params()) if system == "bssn" else (z4, abi.z4_params())
+    rhs = bssn.bssn_rhs_movpunc_N if system == "bssn" else z4.z4_rhs_movpunc_N
+    dl = mod.DeviceLevel(lev)
+    u0 = torch.from_numpy(state(lev, system)).cuda()
+    want = u0.clone()
+    for _ in range(3):
+        mod.evolve_rk_rk4(dl, want, 0.05, p)
+    r0, r = torch.zeros_like(u0), torch.zeros_like(u0)
+    rhs(dl, r0, u0, 0.0, u0, p)
+    u = u0.clone()
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    g = capture(streams[0], lambda st: mod.evolve_rk_rk4(dl, u, 0.05, p, st))
+    for _ in range(3):
+        replay([g], streams, 1)
+        for _ in range(4):
+            rhs(dl, r, u0, 0.0, u0, p, streams[1])
+    torch.cuda.synchronize()
+    assert torch.equal(u, want)
+    assert torch.equal(r, r0)
+    del g
+    dl.close()
