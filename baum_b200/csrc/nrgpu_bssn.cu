@@ -925,7 +925,8 @@ struct RhsTurn {
   cudaStream_t st;
   RhsWork none, *w;
   bool step, capturing;
-  RhsTurn(nrgpu_level *L_, cudaStream_t st_, bool step_) : L(L_), st(st_), none(), w(&none), step(step_) {
+  RhsTurn(nrgpu_level *L_, cudaStream_t st_, bool step_, const RhsRun &run)
+      : L(L_), st(st_), none(), w(&none), step(step_) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     capturing = cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone;
     if (capturing) cudaGetLastError();
@@ -937,19 +938,14 @@ struct RhsTurn {
       else cudaGetLastError();
       if (shared() && cudaStreamWaitEvent(st, L->ev_call, 0) != cudaSuccess) cudaDeviceSynchronize();
     }
-    if (may_allocate() && L->parts) nrgpu_level_lists(L, w);
+    if (!capturing && w != &none) nrgpu_level_reserve(L, w, run);
   }
   ~RhsTurn() {
     if (step || capturing) return;
     if (shared() && cudaEventRecord(L->ev_call, st) != cudaSuccess) cudaStreamSynchronize(st);
     L->call_lock->unlock();
   }
-  bool may_allocate() const { return !capturing && w != &none; }
   bool shared() const { return w->lists || w->pad || L->queue; }  // (the queue's counter)
-  // the staging buffer, when a box runs point by point
-  void pad() {
-    if (may_allocate()) nrgpu_level_pad(L, w);
-  }
   RhsTurn(const RhsTurn &) = delete;
 };
 
@@ -970,16 +966,18 @@ static int launch_rhs(nrgpu_level *L, bool step, const CVarPtrs &U, const VarPtr
     NRGPU_CUDA_TRY(cudaStreamWaitEvent(L->side, L->ev_fork, 0));
   }
   if (interior) {
-    RhsTurn turn(L, st, step);
+    const RhsRun run = nrgpu_rhs_run(L, p);
+    RhsTurn turn(L, st, step, run);
     const RhsWork &w = *turn.w;
     for (int b = 0; b < L->nboxes; ++b) {
       const BoxGeo &bx = L->hbox[b];
       if (bx.m < 3 || bx.n < 3 || bx.o < 3) continue;
       const int k0 = max(kb, 1), k1 = min(ke, bx.o - 2);
       if (k1 < k0) continue;
-      if (L->parts && !L->tile) {
-        if (p.order_centered == 4 && nrgpu_bssn_parts_o4(L, w, b, U.p, out.p, pre.p, acc.p, E, p, st, k0, k1)) continue;
-        if (p.order_centered == 6 && nrgpu_bssn_parts_o6(L, w, b, U.p, out.p, pre.p, acc.p, E, p, st, k0, k1)) continue;
+      if (w.lists && nrgpu_two_kernels(run, bx)) {
+        if (p.order_centered == 4) nrgpu_bssn_parts_o4(L, w, b, U.p, out.p, pre.p, acc.p, E, p, st, k0, k1);
+        else nrgpu_bssn_parts_o6(L, w, b, U.p, out.p, pre.p, acc.p, E, p, st, k0, k1);
+        continue;
       }
       if (L->tile && tile_eligible(L, b, U.p, NRGPU_NV, p.order_centered, p.advection_lopsided,
                                    p.advection_lopsided6)) {
@@ -989,7 +987,7 @@ static int launch_rhs(nrgpu_level *L, bool step, const CVarPtrs &U, const VarPtr
         if ((e = launch_bssn_tile(L, b, maps, U, out, pre, acc, E, p, st, k0, k1))) return e;
         continue;
       }
-      turn.pad();  // point by point
+      // point by point
       // the block shape of the level (32 x 4 x 1, or what nrgpu_level_autotune
       // measured fastest for this box); 128 or 256 threads, one point each
       const dim3 blk(L->blk[0], L->blk[1], L->blk[2]);
@@ -1698,10 +1696,13 @@ static int z4_launch(nrgpu_level *L, bool step, const ZCVarPtrs &U, const ZVarPt
     NRGPU_CUDA_TRY(cudaStreamWaitEvent(L->side, L->ev_fork, 0));
   }
   if (interior) {
-    RhsTurn turn(L, st, step);
+    const RhsRun run = nrgpu_rhs_run(L, p);
+    RhsTurn turn(L, st, step, run);
     const RhsWork &w = *turn.w;
-    // all boxes in one persistent launch (nrgpu_level_queue), or one launch per box
-    const int qm = L->queue && !L->parts && (step || !turn.capturing) ? z4_queue_size(L, p) : 0;
+    // point by point, all boxes in one persistent launch (nrgpu_level_queue), or
+    // one launch per box
+    const bool two = w.lists && nrgpu_two_kernels(run, L->hbox[0]);
+    const int qm = L->queue && !two && (step || !turn.capturing) ? z4_queue_size(L, p) : 0;
     if (qm) {
       int e = z4_queue_launch(L, qm, L->d_status + (step ? 2 : 3), U, out, pre, acc, E, p, st);
       if (e) return e;
@@ -1709,12 +1710,11 @@ static int z4_launch(nrgpu_level *L, bool step, const ZCVarPtrs &U, const ZVarPt
     for (int b = 0; b < L->nboxes && !qm; ++b) {
       const BoxGeo &bx = L->hbox[b];
       if (bx.m < 3 || bx.n < 3 || bx.o < 3) continue;
-      if (L->parts && p.precision == 0) {
-        const int k1 = bx.o - 2;
-        if (p.order_centered == 4 && nrgpu_z4_parts_o4(L, w, b, U.p, out.p, pre.p, acc.p, E, p, st, 1, k1)) continue;
-        if (p.order_centered == 6 && nrgpu_z4_parts_o6(L, w, b, U.p, out.p, pre.p, acc.p, E, p, st, 1, k1)) continue;
+      if (w.lists && nrgpu_two_kernels(run, bx)) {
+        if (p.order_centered == 4) nrgpu_z4_parts_o4(L, w, b, U.p, out.p, pre.p, acc.p, E, p, st, 1, bx.o - 2);
+        else nrgpu_z4_parts_o6(L, w, b, U.p, out.p, pre.p, acc.p, E, p, st, 1, bx.o - 2);
+        continue;
       }
-      turn.pad();
       // the block shape of the level (32 x 4 x 1, or what nrgpu_level_autotune
       // measured fastest for this box); 128 or 256 threads, one point each
       const dim3 blk(L->blk[0], L->blk[1], L->blk[2]);
@@ -1903,20 +1903,16 @@ extern "C" int nrgpu_level_autotune(nrgpu_level *L, int system, const void *para
                                 {64, 2, 2}, {128, 2, 1}};
   const int ncand = (int)(sizeof cand / sizeof cand[0]);
   // the two kernels of nrgpu_deriv.cuh take their tiles from the box: where
-  // they run, no shape is timed and the level's stays.  (They beat the
-  // staged tiles on every box: 66^3 0.21 against 0.27 ms.)
-  bool parts;
-  if (system == NRGPU_SYSTEM_BSSN) {
-    const nrgpu_bssn_params &q = *(const nrgpu_bssn_params *)params;
-    parts = nrgpu_parts_cover(q.order_centered, q.advection_lopsided, q.advection_lopsided6);
-  } else {
-    const nrgpu_z4_params &q = *(const nrgpu_z4_params *)params;
-    parts = q.precision == 0 && nrgpu_parts_cover(q.order_centered, q.advection_lopsided, q.advection_lopsided6);
-  }
-  for (int b = 0; b < L->nboxes; ++b)
-    parts = parts && (long)L->hbox[b].m * L->hbox[b].n * L->hbox[b].o >= 2 * NRGPU_PARTS_MIN_POINTS;
-  if (parts && L->parts && L->step_work.lists) {
-    L->tile = 0;
+  // they run on every box, no shape is timed and the level's stays; where
+  // they run on one, neither staged tiles nor the queue take their place.
+  // (They beat the staged tiles on every box: 66^3 0.21 against 0.27 ms.)
+  L->tile = L->queue = 0;
+  const RhsRun run = system == NRGPU_SYSTEM_BSSN ? nrgpu_rhs_run(L, *(const nrgpu_bssn_params *)params)
+                                                 : nrgpu_rhs_run(L, *(const nrgpu_z4_params *)params);
+  nrgpu_level_reserve(L, &L->step_work, run);
+  int two = 0;
+  for (int b = 0; b < L->nboxes && L->step_work.lists; ++b) two += nrgpu_two_kernels(run, L->hbox[b]);
+  if (two == L->nboxes) {
     for (int q = 0; q < 3; ++q)
       if (best_block) best_block[q] = L->blk[q];
     cudaEventDestroy(ev0);
@@ -1957,8 +1953,7 @@ extern "C" int nrgpu_level_autotune(nrgpu_level *L, int system, const void *para
   }
   for (int q = 0; q < 3; ++q) L->blk[q] = cand[bb][q];
   // the staged-tile kernel (BSSN) against the fastest shape
-  L->tile = 0;
-  if (!e && system == NRGPU_SYSTEM_BSSN) {
+  if (!e && !two && system == NRGPU_SYSTEM_BSSN) {
     const nrgpu_bssn_params &bp = *(const nrgpu_bssn_params *)params;
     VarPtrs P, O;
     for (int v = 0; v < NRGPU_NV; ++v) {
@@ -1989,8 +1984,7 @@ extern "C" int nrgpu_level_autotune(nrgpu_level *L, int system, const void *para
   }
   // the box work-queue kernel (Z4c levels of several equal boxes) against
   // one launch per box with the fastest shape
-  L->queue = 0;
-  if (!e && system == NRGPU_SYSTEM_Z4C && z4_queue_size(L, *(const nrgpu_z4_params *)params)) {
+  if (!e && !two && system == NRGPU_SYSTEM_Z4C && z4_queue_size(L, *(const nrgpu_z4_params *)params)) {
     const nrgpu_z4_params &zp = *(const nrgpu_z4_params *)params;
     ZVarPtrs P, O;
     for (int v = 0; v < ZNV; ++v) {

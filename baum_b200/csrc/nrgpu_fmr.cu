@@ -646,6 +646,13 @@ void launch_prolong(const Ptrs &uc, const Ptrs &uf, const Box3 &cb, const Box3 &
   prolong_kernel<N><<<dim3((n + 127) / 128, nv), 128, 0, st>>>(uc, uf, cb, fb, G, list, n);
 }
 
+// the rhs workspace of level l's steps: a graph may be captured before the
+// first eager step of a level (after a regrid, after nrgpu_fmr_load)
+void reserve_steps(const nrgpu_fmr *F, int l, nrgpu_level *L) {
+  nrgpu_level_reserve(L, &L->step_work,
+                      F->p.system == NRGPU_SYSTEM_BSSN ? nrgpu_rhs_run(L, F->bp[l]) : nrgpu_rhs_run(L, F->zp[l]));
+}
+
 int regrid_level(nrgpu_fmr *F, int m, const nrgpu_level_desc &d, double *const *uold, double *const *unew,
                  double *const *uparent, cudaStream_t st) {
   if (d.symmetry) return nrgpu_set_error(NRGPU_ERR_UNSUPPORTED, "level %d: symmetry grids", m);
@@ -670,6 +677,7 @@ int regrid_level(nrgpu_fmr *F, int m, const nrgpu_level_desc &d, double *const *
     nrgpu_level_destroy(nL);
     return e;
   }
+  reserve_steps(F, m, nL);
   int blk[3];
   if (!nrgpu_level_get_block(oL, blk)) nrgpu_level_block(nL, blk[0], blk[1], blk[2]);
   nL->parts = oL->parts;
@@ -924,6 +932,7 @@ extern "C" int nrgpu_fmr_create(int nl, const nrgpu_level_desc *levels, const do
                                   p->system == NRGPU_SYSTEM_BSSN ? (const void *)&F->bp[l] : (const void *)&F->zp[l],
                                   nullptr, nullptr)))
       break;
+    reserve_steps(F, l, F->L[l]);
     if (l < nl - 1) {
       const size_t bytes = sizeof(double) * F->nv * (size_t)d.npoints;
       if (cudaMalloc(&F->up[l], bytes) != cudaSuccess || cudaMalloc(&F->upp[l], bytes) != cudaSuccess) {

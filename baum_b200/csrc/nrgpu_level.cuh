@@ -136,7 +136,7 @@ int nrgpu_z4_rk4_background(nrgpu_level *L, double *const *u, double dt, const n
 int nrgpu_level_scratch(nrgpu_level *L, double **out);
 // the box sizes with a compile-time-stride Z4c rhs kernel; a box of another
 // size up to the largest is staged into a copy with the strides of the next
-// one (nrgpu_level_pad)
+// one (nrgpu_level_reserve)
 constexpr int kPadSizes[] = {66, 72, 104, 136, 162, 168, 194};
 // the staging size of an m x n box: 0 when it has a kernel of its own or is
 // too large
@@ -148,31 +148,58 @@ inline int nrgpu_pad_size(int m, int n) {
     if (c >= m && c >= n) return c;
   return 0;
 }
-void nrgpu_level_pad(const nrgpu_level *L, RhsWork *w);
-// the lists of the two rhs kernels, tried once per workspace; without them
-// the point-by-point kernels run (nrgpu_lib.cu)
+// sizes of the lists of the two rhs kernels
 #define NRGPU_DERIV_LISTS 71
 #define NRGPU_DERIV_PITCH 128
 #define NRGPU_PARTS_MIN_POINTS 50000
 #define NRGPU_PARTS_MAX_LEVELS 5
-void nrgpu_level_lists(const nrgpu_level *L, RhsWork *w);
-// whether those kernels have the run's advection rows: shifts 1 and 2
-// (centred) at 4th order, 2 and 3 (centred) at 6th
-inline bool nrgpu_parts_cover(int order, int lop, int lop6) {
+// what a run's parameters allow on a level: the two kernels (FP64, advection
+// rows shifted by 1 or 2 (centred) at 4th order, by 2 or 3 (centred) at 6th; a
+// BSSN level whose staged tiles are switched on takes those), and a staging
+// copy for the point-by-point kernels
+struct RhsRun {
+  int order;
+  bool two, staged;
+};
+inline bool nrgpu_two_kernels_rows(int order, int lop, int lop6) {
   return order == 4 ? lop == 1 || lop == 2 : order == 6 && (lop6 == 2 || lop6 == 3);
 }
+inline RhsRun nrgpu_rhs_run(const nrgpu_level *L, const nrgpu_bssn_params &p) {
+  return {p.order_centered,
+          L->parts && !L->tile && nrgpu_two_kernels_rows(p.order_centered, p.advection_lopsided, p.advection_lopsided6),
+          p.order_centered >= 4};
+}
+inline RhsRun nrgpu_rhs_run(const nrgpu_level *L, const nrgpu_z4_params &p) {
+  return {p.order_centered,
+          L->parts && p.precision == 0 &&
+              nrgpu_two_kernels_rows(p.order_centered, p.advection_lopsided, p.advection_lopsided6),
+          p.order_centered >= 4 && p.precision == 0};
+}
+// whether a run takes the two kernels on a box, given their lists: the one
+// rule of the launches, the allocation and the tuner.  Small boxes leave most
+// SMs idle either way, and one launch is cheaper than two: 34^3 step 217 us
+// point by point against 222, 50^3 774 against 563
+inline bool nrgpu_two_kernels(const RhsRun &run, const BoxGeo &b) {
+  const int f = run.order;  // two faces of order / 2 points
+  return run.two && b.m > f && b.n > f && b.o > f &&
+         (long)(b.m - f) * (b.n - f) * (b.o - f) >= NRGPU_PARTS_MIN_POINTS;
+}
+// what the run uses of a workspace: the lists, and the staging buffer where a
+// box goes point by point; each allocated once, and without memory for them
+// the point-by-point kernels run, at run-time strides (nrgpu_lib.cu)
+void nrgpu_level_reserve(const nrgpu_level *L, RhsWork *w, const RhsRun &run);
 // interior rhs of box b on planes kb .. ke by those kernels, per system and
-// order, with the lists of w; false when they do not apply (nrgpu_parts_*.cu)
-bool nrgpu_bssn_parts_o4(nrgpu_level *L, const RhsWork &w, int b, const double *const *U, double *const *out,
+// order, with the lists of w, where nrgpu_two_kernels holds (nrgpu_parts_*.cu)
+void nrgpu_bssn_parts_o4(nrgpu_level *L, const RhsWork &w, int b, const double *const *U, double *const *out,
                          const double *const *pre, double *const *acc, const Epilogue &E, const nrgpu_bssn_params &p,
                          cudaStream_t st, int kb, int ke);
-bool nrgpu_bssn_parts_o6(nrgpu_level *L, const RhsWork &w, int b, const double *const *U, double *const *out,
+void nrgpu_bssn_parts_o6(nrgpu_level *L, const RhsWork &w, int b, const double *const *U, double *const *out,
                          const double *const *pre, double *const *acc, const Epilogue &E, const nrgpu_bssn_params &p,
                          cudaStream_t st, int kb, int ke);
-bool nrgpu_z4_parts_o4(nrgpu_level *L, const RhsWork &w, int b, const double *const *U, double *const *out,
+void nrgpu_z4_parts_o4(nrgpu_level *L, const RhsWork &w, int b, const double *const *U, double *const *out,
                        const double *const *pre, double *const *acc, const Epilogue &E, const nrgpu_z4_params &p,
                        cudaStream_t st, int kb, int ke);
-bool nrgpu_z4_parts_o6(nrgpu_level *L, const RhsWork &w, int b, const double *const *U, double *const *out,
+void nrgpu_z4_parts_o6(nrgpu_level *L, const RhsWork &w, int b, const double *const *U, double *const *out,
                        const double *const *pre, double *const *acc, const Epilogue &E, const nrgpu_z4_params &p,
                        cudaStream_t st, int kb, int ke);
 // set_boundary_symmetry on a list of nv variables of the given system

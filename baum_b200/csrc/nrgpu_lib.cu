@@ -224,44 +224,43 @@ extern "C" int nrgpu_level_destroy(nrgpu_level *L) {
   return NRGPU_OK;
 }
 
+// The lists that the two rhs kernels pass from one to the other, for as many
+// rows of a part of the largest box that takes them as kListBytes hold; and
 // the staging buffer for boxes of up to 194 points per side without a
 // compile-time-stride kernel of their own: 25 lists with strides (1, P, P P),
-// P the next kernel size (kPadSizes); tried once per workspace, and without it
-// those boxes run the run-time-stride kernel
-void nrgpu_level_pad(const nrgpu_level *L, RhsWork *w) {
-  if (w->pad_tried) return;
-  w->pad_tried = 1;
-  size_t need = 0;
-  for (int b = 0; b < L->nboxes; ++b) {
-    const int P = nrgpu_pad_size(L->hbox[b].m, L->hbox[b].n);
-    if (P > 0) need = std::max(need, (size_t)NRGPU_Z4_NVARS * P * P * L->hbox[b].o);
-  }
-  if (need && cudaMalloc(&w->pad, sizeof(double) * need) == cudaSuccess) {
-    w->pad_doubles = need;
-  } else {
-    cudaGetLastError();
-    w->pad = nullptr;
-    w->pad_doubles = 0;
-  }
-}
-
-// The lists that the two rhs kernels pass from one to the other, for as many
-// rows of a part of the largest box as kListBytes hold.
+// P the next kernel size (kPadSizes).
 constexpr size_t kListBytes = (size_t)512 << 20;
-void nrgpu_level_lists(const nrgpu_level *L, RhsWork *w) {
-  if (w->lists_tried) return;
-  w->lists_tried = 1;
+void nrgpu_level_reserve(const nrgpu_level *L, RhsWork *w, const RhsRun &run) {
   constexpr size_t row = sizeof(double) * NRGPU_DERIV_LISTS * NRGPU_DERIV_PITCH;
   size_t rows = 0;
-  for (int b = 0; b < L->nboxes; ++b)
-    if ((long)L->hbox[b].m * L->hbox[b].n * L->hbox[b].o >= NRGPU_PARTS_MIN_POINTS)
-      rows = std::max(rows, (size_t)L->hbox[b].n * std::max(0, L->hbox[b].o - 4));
-  rows = std::min(rows, kListBytes / row);
-  if (rows && cudaMalloc(&w->lists, rows * row) == cudaSuccess) {
-    w->list_rows = rows;
-  } else {
-    cudaGetLastError();
-    w->lists = nullptr;
+  for (int b = 0; b < L->nboxes && !w->lists_tried; ++b)
+    if (nrgpu_two_kernels(run, L->hbox[b])) rows = std::max(rows, (size_t)L->hbox[b].n * (L->hbox[b].o - 4));
+  if (rows) {
+    w->lists_tried = 1;
+    rows = std::min(rows, kListBytes / row);
+    if (cudaMalloc(&w->lists, rows * row) == cudaSuccess) {
+      w->list_rows = rows;
+    } else {
+      cudaGetLastError();
+      w->lists = nullptr;
+    }
+  }
+  bool pad = false;
+  size_t need = 0;
+  for (int b = 0; b < L->nboxes && run.staged && !w->pad_tried; ++b) {
+    const int P = nrgpu_pad_size(L->hbox[b].m, L->hbox[b].n);
+    if (P == 0) continue;
+    pad = pad || !(w->lists && nrgpu_two_kernels(run, L->hbox[b]));
+    need = std::max(need, (size_t)NRGPU_Z4_NVARS * P * P * L->hbox[b].o);
+  }
+  if (pad) {
+    w->pad_tried = 1;
+    if (cudaMalloc(&w->pad, sizeof(double) * need) == cudaSuccess) {
+      w->pad_doubles = need;
+    } else {
+      cudaGetLastError();
+      w->pad = nullptr;
+    }
   }
 }
 
@@ -276,8 +275,6 @@ int nrgpu_level_scratch(nrgpu_level *L, double **out) {
       return nrgpu_set_error(NRGPU_ERR_NOMEM, "RK4 scratch of %zu bytes", bytes);
     }
     L->scratch_points = (size_t)L->npoints;
-    if (L->parts) nrgpu_level_lists(L, &L->step_work);
-    if (!L->step_work.lists) nrgpu_level_pad(L, &L->step_work);
   }
   *out = L->scratch;
   return NRGPU_OK;

@@ -50,8 +50,6 @@ void launch_algebra(const CPtrs<NV> &U, const AlgebraGeo &g, const SinkArgs<NV> 
   else algebra_kernel<ORD, NV, EPI_ADDLINEAR><<<grd, kAlgebraThreads, 0, st>>>(U, g, sa, p, status);
 }
 
-constexpr long kPartsMinPoints = NRGPU_PARTS_MIN_POINTS;
-
 // n points cut into the fewest equal parts of at most `most`
 int part_size(int n, int most) {
   const int parts = (n + most - 1) / most;
@@ -59,22 +57,17 @@ int part_size(int n, int most) {
 }
 
 // interior rhs of box b on planes kb .. ke by the two kernels of
-// nrgpu_deriv.cuh, part by part; false when they do not apply (nothing
-// launched then)
+// nrgpu_deriv.cuh, part by part
 template <int NV, int ORD, class PARAMS>
-bool launch_parts(nrgpu_level *L, const RhsWork &w, int b, const double *const *U, double *const *out,
+void launch_parts(nrgpu_level *L, const RhsWork &w, int b, const double *const *U, double *const *out,
                   const double *const *pre, double *const *acc, const Epilogue &E, const PARAMS &p, cudaStream_t st,
                   int kb, int ke) {
   constexpr int H = ORD / 2;
   const int lop = ORD == 4 ? p.advection_lopsided : p.advection_lopsided6;
-  if (!nrgpu_parts_cover(ORD, p.advection_lopsided, p.advection_lopsided6) || w.list_rows <= 2 * H) return false;
   const BoxGeo &bx = L->hbox[b];
   const int z0 = std::max(kb, H), z1 = std::min(ke, bx.o - 1 - H);
   const int nx = bx.m - 2 * H, ny = bx.n - 2 * H, nz = z1 - z0 + 1;
-  if (nx < 1 || ny < 1 || nz < 1) return true;  // ladder points only
-  // small boxes leave most SMs idle either way, and one launch is cheaper than
-  // two: 34^3 step 217 us point by point against 222, 50^3 774 against 563
-  if ((long)nx * ny * (bx.o - 2 * H) < kPartsMinPoints) return false;
+  if (nz < 1) return;  // ladder points only
   const size_t rows = w.list_rows;
   const int px = part_size(nx, kPartX);
   const int py = part_size(ny, (int)std::min<size_t>(rows - 2 * H, ny));
@@ -131,7 +124,6 @@ bool launch_parts(nrgpu_level *L, const RhsWork &w, int b, const double *const *
         g.tiles_x = (wx + g.w - 1) / g.w;
         launch_algebra<NV, ORD>(cu, g, sa, p, E.mode, L->d_status, st);
       }
-  return true;
 }
 
 }  // namespace

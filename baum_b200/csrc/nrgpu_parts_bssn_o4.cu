@@ -1,8 +1,8 @@
 // nrgpu_parts_bssn_o4.cu -- the two rhs kernels for BSSN, order 4.
 #include "nrgpu_parts.cuh"
 
-bool nrgpu_bssn_parts_o4(nrgpu_level *L, const RhsWork &w, int b, const double *const *U, double *const *out,
+void nrgpu_bssn_parts_o4(nrgpu_level *L, const RhsWork &w, int b, const double *const *U, double *const *out,
                          const double *const *pre, double *const *acc, const Epilogue &E, const nrgpu_bssn_params &p,
                          cudaStream_t st, int kb, int ke) {
-  return launch_parts<NRGPU_NV, 4>(L, w, b, U, out, pre, acc, E, p, st, kb, ke);
+  launch_parts<NRGPU_NV, 4>(L, w, b, U, out, pre, acc, E, p, st, kb, ke);
 }

@@ -1,8 +1,8 @@
 // nrgpu_parts_z4_o4.cu -- the two rhs kernels for Z4c, order 4.
 #include "nrgpu_parts.cuh"
 
-bool nrgpu_z4_parts_o4(nrgpu_level *L, const RhsWork &w, int b, const double *const *U, double *const *out,
+void nrgpu_z4_parts_o4(nrgpu_level *L, const RhsWork &w, int b, const double *const *U, double *const *out,
                        const double *const *pre, double *const *acc, const Epilogue &E, const nrgpu_z4_params &p,
                        cudaStream_t st, int kb, int ke) {
-  return launch_parts<NRGPU_Z4_NVARS, 4>(L, w, b, U, out, pre, acc, E, p, st, kb, ke);
+  launch_parts<NRGPU_Z4_NVARS, 4>(L, w, b, U, out, pre, acc, E, p, st, kb, ke);
 }

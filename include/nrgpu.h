@@ -497,7 +497,9 @@ enum { NRGPU_SYSTEM_BSSN = 0, NRGPU_SYSTEM_Z4C = 1 };
  * Boxes of at least 50000 inner points run their 4th- and 6th-order interior
  * rhs in two kernels that choose their own tiles (advection shifts 1 and 2 at
  * 4th order, 2 and 3 at 6th; FP64; not on the levels of a hierarchy deeper
- * than five): there nothing is timed and the level's shape stays.  Their
+ * than five, nor where nrgpu_level_tile is on): where every box does, nothing is
+ * timed and the level's shape stays, and where one does, neither staged tiles
+ * nor the queue are tried.  Their
  * intermediate lists take up to 512 MB per level for the RK steps and as much
  * again for nrgpu_bssn_rhs and nrgpu_z4_rhs, each allocated on its first use
  * outside a graph capture.  rhs calls of one level may overlap (host threads,
@@ -533,10 +535,10 @@ int nrgpu_level_tile(nrgpu_level *L, int on);
 /* The Z4c interior rhs of all boxes of a level in one persistent launch:
  * the blocks take tiles from a queue over the boxes (an atomic counter)
  * until it is empty, each point computed as by the per-box kernel, so the
- * results are identical.  For levels of a hierarchy deeper than five that
- * have two or more boxes of one size with a compile-time-stride kernel (66,
- * 72, 104, 136, 162, 168, 194 points in x and y), 4th or 6th order, FP64; one
- * launch per box otherwise.
+ * results are identical.  For levels whose run goes point by point (see
+ * nrgpu_level_autotune) and that have two or more boxes of one size with a
+ * compile-time-stride kernel (66, 72, 104, 136, 162, 168, 194 points in x and
+ * y), 4th or 6th order, FP64; one launch per box otherwise.
  * on = 1 on, 0 off, -1 only queries; returns the setting.
  * nrgpu_level_autotune turns it on where it measures faster.  No
  * counterpart in the reference (advance_levelandsublevels, main.c:397-418,

@@ -177,3 +177,55 @@ def test_captured_step_is_the_eager_step(gpu, system):
     assert torch.equal(r, r0)
     del g
     dl.close()
+
+
+def held_by(fn):
+    """Device memory in MB that fn leaves allocated outside torch's pool."""
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    fn()
+    torch.cuda.synchronize()
+    return (free - torch.cuda.mem_get_info()[0]) / 2 ** 20
+
+
+@pytest.mark.parametrize("shape,over,lists", [
+    ((38, 38, 38), {}, False),                                             # 50000 points, but not inner ones
+    ((42, 41, 42), {}, True),                                              # 38 x 37 x 38 inner
+    ((42, 41, 42), {"order_centered": 6, "order_advection": 6}, False),    # 36 x 35 x 36 inner
+    ((7, 130, 130), {}, False),                                            # 118300 points, 3 x 126 x 126 inner
+    ((72, 72, 72), {"order_centered": 2, "order_advection": 2}, False),
+    ((72, 72, 72), {"precision": 1}, False),
+    ((72, 72, 72), {"advection_lopsided": 0}, False),
+])
+def test_lists_are_held_where_the_two_kernels_run(gpu, shape, over, lists):
+    """The lists of a level (71 x 128 doubles per row of its largest box) are
+    allocated by one rule with the launches: 50000 inner points, and a run
+    that the kernels cover."""
+    lev = box(*shape)
+    p = abi.z4_params(**over)
+    u = torch.from_numpy(state(lev, "z4")).cuda()
+    r = torch.zeros_like(u)
+    dl = z4.DeviceLevel(lev)
+    z4.z4_rhs_movpunc_N(dl, r, u, 0.0, u, p)   # the kernels' own memory
+    dl.close()
+    dl = z4.DeviceLevel(lev)
+    side = min([c for c in (66, 72, 136) if c >= max(shape[:2])])
+    other = 25 * side * side * shape[2] * 8 / 2 ** 20 if side != shape[0] else 0   # a staging copy
+    size = 71 * 128 * 8 * shape[1] * (shape[2] - 4) / 2 ** 20
+    got = held_by(lambda: z4.z4_rhs_movpunc_N(dl, r, u, 0.0, u, p))
+    assert (size - 4 < got < size + 8) if lists else got < other + 8, (got, size, other)
+    dl.close()
+
+
+def test_tuner_leaves_the_shape_where_the_two_kernels_run(gpu):
+    """From 50000 inner points nothing is timed; below, a shape is."""
+    dl = z4.DeviceLevel(box(42, 41, 42))
+    dl.set_block(4, 4, 8)
+    assert dl.autotune(abi.SYSTEM_Z4C, abi.z4_params()) == (4, 4, 8)
+    dl.close()
+    dl = bssn.DeviceLevel(box(42, 41, 42))
+    dl.set_block(4, 4, 8)
+    dl.tile(1)
+    assert dl.autotune(abi.SYSTEM_BSSN, abi.bssn_params()) == (4, 4, 8)
+    assert dl.tile() == 0
+    dl.close()
