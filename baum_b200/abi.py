@@ -216,6 +216,8 @@ class FmrParams(C.Structure):
 
 
 SYSTEM_BSSN, SYSTEM_Z4C = 0, 1
+# the kernels of an interior rhs (NRGPU_ROUTE_*)
+ROUTES = ("point", "staged", "parts", "tile", "queue")
 
 
 def fmr_params(**over):
@@ -354,6 +356,7 @@ def lib():
         "nrgpu_fmr_advance": (C.c_int, [vp, pp, C.c_int, vp]),
         "nrgpu_fmr_iteration": (C.c_int, [vp, C.c_int]),
         "nrgpu_fmr_block": (C.c_int, [vp, C.c_int, C.POINTER(C.c_int)]),
+        "nrgpu_fmr_route": (C.c_int, [vp, C.c_int, C.c_int]),
         "nrgpu_fmr_state_size": (C.c_int, [vp, C.POINTER(C.c_size_t)]),
         "nrgpu_fmr_save": (C.c_int, [vp, vp, C.c_size_t]),
         "nrgpu_fmr_load": (C.c_int, [vp, vp, C.c_size_t]),
@@ -379,6 +382,8 @@ def lib():
         "nrgpu_level_block": (C.c_int, [vp, C.c_int, C.c_int, C.c_int]),
         "nrgpu_level_get_block": (C.c_int, [vp, C.POINTER(C.c_int)]),
         "nrgpu_level_tile": (C.c_int, [vp, C.c_int]),
+        "nrgpu_level_parts": (C.c_int, [vp, C.c_int]),
+        "nrgpu_level_route": (C.c_int, [vp, C.c_int, vp, C.c_int]),
         "nrgpu_level_queue": (C.c_int, [vp, C.c_int]),
         "nrgpu_puncture_coefficients": (C.c_int, [C.c_int, C.c_double, C.c_int, C.POINTER(C.c_double),
                                                   C.POINTER(C.c_double), C.POINTER(C.c_double),

@@ -83,6 +83,23 @@ class DeviceLevel:
             abi.check(r)
         return int(r)
 
+    def parts(self, on=-1):
+        """The interior rhs in two kernels where they cover the run
+        (nrgpu_level_parts): on = 1, 0 (point by point), or -1 to query."""
+        r = abi.lib().nrgpu_level_parts(self.handle, int(on))
+        if r < 0:
+            abi.check(r)
+        return int(r)
+
+    def route(self, params, box=0):
+        """The kernels of the next RK step's interior rhs on a box
+        (nrgpu_level_route): one of abi.ROUTES."""
+        system = abi.SYSTEM_BSSN if isinstance(params, abi.BssnParams) else abi.SYSTEM_Z4C
+        r = abi.lib().nrgpu_level_route(self.handle, system, C.byref(params), int(box))
+        if r < 0:
+            abi.check(r)
+        return abi.ROUTES[r]
+
     def tile(self, on=-1):
         """The staged-tile (TMA) interior rhs: on = 1 (a block per tile), 2
         (persistent), 0 (off); -1 only queries; returns the setting."""

@@ -949,6 +949,21 @@ struct RhsTurn {
   RhsTurn(const RhsTurn &) = delete;
 };
 
+// whether box b is staged into the workspace's copy at order 4 or 6
+static bool staged_box(const RhsWork &w, const RhsRun &run, int nv, const BoxGeo &bx) {
+  const size_t Q = run.staged ? nrgpu_pad_size(bx.m, bx.n) : 0;
+  return Q && w.pad && nv * Q * Q * bx.o <= w.pad_doubles;
+}
+
+// the kernels of box b's interior (NRGPU_ROUTE_*)
+static int bssn_route(const nrgpu_level *L, const RhsWork &w, const RhsRun &run, int b, const double *const *U,
+                      const nrgpu_bssn_params &p) {
+  if (w.lists && nrgpu_two_kernels(run, L->hbox[b])) return NRGPU_ROUTE_PARTS;
+  if (L->tile && tile_eligible(L, b, U, NRGPU_NV, p.order_centered, p.advection_lopsided, p.advection_lopsided6))
+    return NRGPU_ROUTE_TILE;
+  return staged_box(w, run, NRGPU_NV, L->hbox[b]) ? NRGPU_ROUTE_STAGED : NRGPU_ROUTE_POINT;
+}
+
 // launch the interior and flagged kernels of one rhs evaluation
 // (step: of an RK step, see RhsTurn; kb <= k <= ke: the planes of the
 // interior launch, whole boxes by default)
@@ -974,13 +989,13 @@ static int launch_rhs(nrgpu_level *L, bool step, const CVarPtrs &U, const VarPtr
       if (bx.m < 3 || bx.n < 3 || bx.o < 3) continue;
       const int k0 = max(kb, 1), k1 = min(ke, bx.o - 2);
       if (k1 < k0) continue;
-      if (w.lists && nrgpu_two_kernels(run, bx)) {
+      const int route = bssn_route(L, w, run, b, U.p, p);
+      if (route == NRGPU_ROUTE_PARTS) {
         if (p.order_centered == 4) nrgpu_bssn_parts_o4(L, w, b, U.p, out.p, pre.p, acc.p, E, p, st, k0, k1);
         else nrgpu_bssn_parts_o6(L, w, b, U.p, out.p, pre.p, acc.p, E, p, st, k0, k1);
         continue;
       }
-      if (L->tile && tile_eligible(L, b, U.p, NRGPU_NV, p.order_centered, p.advection_lopsided,
-                                   p.advection_lopsided6)) {
+      if (route == NRGPU_ROUTE_TILE) {
         const CUtensorMap *maps = nullptr;
         int e = tma_maps(L, b, U.p, NRGPU_NV, &maps);
         if (e) return e;
@@ -1001,22 +1016,17 @@ static int launch_rhs(nrgpu_level *L, bool step, const CVarPtrs &U, const VarPtr
       CVarPtrs In = U;
       int3 in = make_int3(bx.noffset, bx.m, bx.n);
       int P = ord >= 4 && bx.m == bx.n ? bx.m : 0;
-      const int Q = ord >= 4 ? nrgpu_pad_size(bx.m, bx.n) : 0;
-      if (Q && w.pad) {
-        const long fs = (long)Q * Q * bx.o;
-        P = 0;
-        if ((size_t)(NRGPU_NV * fs) <= w.pad_doubles) {
-          // the planes the launch's stencils reach (a launch on some planes:
-          // the host-buffer step's slabs)
-          const int H = max(max(p.order_advection, p.order_centered / 2 + 1), p.order_dissipation / 2 + 1);
-          const int klo = max(0, k0 - H), khi = min(bx.o - 1, k1 + H);
-          const long nb = (long)bx.m * bx.n * (khi - klo + 1);
-          pad_copy_kernel<<<dim3((unsigned)((nb + 255) / 256), NRGPU_NV), 256, 0, st>>>(U, w.pad, bx, Q, fs, klo,
-                                                                                        khi);
-          for (int v = 0; v < NRGPU_NV; ++v) In.p[v] = w.pad + v * fs;
-          in = make_int3(0, Q, Q);
-          P = Q;
-        }
+      if (route == NRGPU_ROUTE_STAGED) {
+        P = nrgpu_pad_size(bx.m, bx.n);
+        const long fs = (long)P * P * bx.o;
+        // the planes the launch's stencils reach (a launch on some planes:
+        // the host-buffer step's slabs)
+        const int H = max(max(p.order_advection, p.order_centered / 2 + 1), p.order_dissipation / 2 + 1);
+        const int klo = max(0, k0 - H), khi = min(bx.o - 1, k1 + H);
+        const long nb = (long)bx.m * bx.n * (khi - klo + 1);
+        pad_copy_kernel<<<dim3((unsigned)((nb + 255) / 256), NRGPU_NV), 256, 0, st>>>(U, w.pad, bx, P, fs, klo, khi);
+        for (int v = 0; v < NRGPU_NV; ++v) In.p[v] = w.pad + v * fs;
+        in = make_int3(0, P, P);
       }
 #define NR_BSSN_LDG(CSY_, CSZ_, ORD_)                                                                          \
   bssn_rhs_kernel<CSY_, CSZ_, ORD_><<<grd, blk, 0, st>>>(In, out, pre, acc, E, p, bx, L->d_boundary, L->dx, L->dy, \
@@ -1584,15 +1594,15 @@ static ZCVarPtrs z4_c(const ZVarPtrs &v) {
 // FP64 interior launch with compile-time strides for the box sizes of the
 // workloads (66, 162, the finer levels of the batched refinement step, and
 // 194, the coarsest level of the full form's grid).  A box of another size
-// up to 194 points per side is staged first into the level's padding
-// buffer with the strides of the next such size (nrgpu_level_pad), whose
-// kernel then reads it: with run-time strides the kernel's tap addresses
+// up to 194 points per side is staged first into the workspace's padding
+// buffer (pad, null where the box is not staged) with the strides of the next
+// such size, whose kernel then reads it: with run-time strides the kernel's tap addresses
 // take registers of their own, it spills, and it runs about half as fast.
 // Generic strides remain for larger boxes; one kernel per stencil order.
 template <int ORD>
 static void z4_interior_fp64(const ZCVarPtrs &U, const ZVarPtrs &out, const ZCVarPtrs &pre, const ZVarPtrs &acc,
                              const Epilogue &E, const nrgpu_z4_params &p, const BoxGeo &bx, nrgpu_level *L,
-                             const RhsWork &w, dim3 grd, dim3 blk, cudaStream_t st) {
+                             double *pad, dim3 grd, dim3 blk, cudaStream_t st) {
 #define NRGPU_Z4_FIXED(M_)                                                                                   \
   if (P == M_) {                                                                                             \
     z4_rhs_kernel<M_, M_ * M_, 0, ORD><<<grd, blk, 0, st>>>(In, out, pre, acc, E, p, bx, L->d_boundary, L->dx, \
@@ -1603,19 +1613,13 @@ static void z4_interior_fp64(const ZCVarPtrs &U, const ZVarPtrs &out, const ZCVa
     ZCVarPtrs In = U;
     int3 in = make_int3(bx.noffset, bx.m, bx.n);
     int P = bx.m == bx.n ? bx.m : 0;  // a kernel of its own, if one below matches
-    const int Q = nrgpu_pad_size(bx.m, bx.n);
-    if (Q && w.pad) {
-      P = Q;
-      const long fs = (long)P * P * bx.o;
-      if ((size_t)(NRGPU_Z4_NVARS * fs) <= w.pad_doubles) {
-        const long nb = (long)bx.m * bx.n * bx.o;
-        pad_copy_kernel<<<dim3((unsigned)((nb + 255) / 256), NRGPU_Z4_NVARS), 256, 0, st>>>(U, w.pad, bx, P, fs, 0,
-                                                                                              bx.o - 1);
-        for (int v = 0; v < NRGPU_Z4_NVARS; ++v) In.p[v] = w.pad + v * fs;
-        in = make_int3(0, P, P);
-      } else {
-        P = 0;
-      }
+    if (pad) {
+      P = nrgpu_pad_size(bx.m, bx.n);
+      const long fs = (long)P * P * bx.o, nb = (long)bx.m * bx.n * bx.o;
+      pad_copy_kernel<<<dim3((unsigned)((nb + 255) / 256), NRGPU_Z4_NVARS), 256, 0, st>>>(U, pad, bx, P, fs, 0,
+                                                                                            bx.o - 1);
+      for (int v = 0; v < NRGPU_Z4_NVARS; ++v) In.p[v] = pad + v * fs;
+      in = make_int3(0, P, P);
     }
     NRGPU_Z4_FIXED(162) NRGPU_Z4_FIXED(168) NRGPU_Z4_FIXED(136) NRGPU_Z4_FIXED(104) NRGPU_Z4_FIXED(72)
     NRGPU_Z4_FIXED(66) NRGPU_Z4_FIXED(194)
@@ -1684,6 +1688,14 @@ static int z4_queue_launch(nrgpu_level *L, int m, int *counter, const ZCVarPtrs 
   return NRGPU_OK;
 }
 
+// queue: the kernel's counter is free
+static int z4_route(const nrgpu_level *L, const RhsWork &w, const RhsRun &run, int b, const nrgpu_z4_params &p,
+                    bool queue) {
+  if (w.lists && nrgpu_two_kernels(run, L->hbox[b])) return NRGPU_ROUTE_PARTS;
+  if (L->queue && queue && z4_queue_size(L, p)) return NRGPU_ROUTE_QUEUE;
+  return staged_box(w, run, NRGPU_Z4_NVARS, L->hbox[b]) ? NRGPU_ROUTE_STAGED : NRGPU_ROUTE_POINT;
+}
+
 static int z4_launch(nrgpu_level *L, bool step, const ZCVarPtrs &U, const ZVarPtrs &out, const ZCVarPtrs &pre,
                      const ZVarPtrs &acc, const Epilogue &E, const nrgpu_z4_params &p, cudaStream_t st, bool interior,
                      bool flagged) {
@@ -1699,18 +1711,16 @@ static int z4_launch(nrgpu_level *L, bool step, const ZCVarPtrs &U, const ZVarPt
     const RhsRun run = nrgpu_rhs_run(L, p);
     RhsTurn turn(L, st, step, run);
     const RhsWork &w = *turn.w;
-    // point by point, all boxes in one persistent launch (nrgpu_level_queue), or
-    // one launch per box
-    const bool two = w.lists && nrgpu_two_kernels(run, L->hbox[0]);
-    const int qm = L->queue && !two && (step || !turn.capturing) ? z4_queue_size(L, p) : 0;
-    if (qm) {
-      int e = z4_queue_launch(L, qm, L->d_status + (step ? 2 : 3), U, out, pre, acc, E, p, st);
-      if (e) return e;
-    }
-    for (int b = 0; b < L->nboxes && !qm; ++b) {
+    for (int b = 0; b < L->nboxes; ++b) {
       const BoxGeo &bx = L->hbox[b];
       if (bx.m < 3 || bx.n < 3 || bx.o < 3) continue;
-      if (w.lists && nrgpu_two_kernels(run, bx)) {
+      const int route = z4_route(L, w, run, b, p, step || !turn.capturing);
+      if (route == NRGPU_ROUTE_QUEUE) {  // all boxes in one persistent launch
+        int e = z4_queue_launch(L, bx.m, L->d_status + (step ? 2 : 3), U, out, pre, acc, E, p, st);
+        if (e) return e;
+        break;
+      }
+      if (route == NRGPU_ROUTE_PARTS) {
         if (p.order_centered == 4) nrgpu_z4_parts_o4(L, w, b, U.p, out.p, pre.p, acc.p, E, p, st, 1, bx.o - 2);
         else nrgpu_z4_parts_o6(L, w, b, U.p, out.p, pre.p, acc.p, E, p, st, 1, bx.o - 2);
         continue;
@@ -1719,11 +1729,12 @@ static int z4_launch(nrgpu_level *L, bool step, const ZCVarPtrs &U, const ZVarPt
       // measured fastest for this box); 128 or 256 threads, one point each
       const dim3 blk(L->blk[0], L->blk[1], L->blk[2]);
       const dim3 grd((bx.m - 2 + blk.x - 1) / blk.x, (bx.n - 2 + blk.y - 1) / blk.y, (bx.o - 2 + blk.z - 1) / blk.z);
+      double *pad = route == NRGPU_ROUTE_STAGED ? w.pad : nullptr;
       if (p.precision == 1) z4_interior_prec<1>(U, out, pre, acc, E, p, bx, L, grd, blk, st);
       else if (p.precision == 2) z4_interior_prec<2>(U, out, pre, acc, E, p, bx, L, grd, blk, st);
-      else if (p.order_centered == 2) z4_interior_fp64<2>(U, out, pre, acc, E, p, bx, L, w, grd, blk, st);
-      else if (p.order_centered == 4) z4_interior_fp64<4>(U, out, pre, acc, E, p, bx, L, w, grd, blk, st);
-      else z4_interior_fp64<6>(U, out, pre, acc, E, p, bx, L, w, grd, blk, st);
+      else if (p.order_centered == 2) z4_interior_fp64<2>(U, out, pre, acc, E, p, bx, L, pad, grd, blk, st);
+      else if (p.order_centered == 4) z4_interior_fp64<4>(U, out, pre, acc, E, p, bx, L, pad, grd, blk, st);
+      else z4_interior_fp64<6>(U, out, pre, acc, E, p, bx, L, pad, grd, blk, st);
     }
     // the ladder points of all boxes (beside the interior kernel)
     const int nlad = L->nladder[p.order_centered / 2 - 1];
@@ -2025,6 +2036,29 @@ extern "C" int nrgpu_level_queue(nrgpu_level *L, int on) {
   if (on > 1) return nrgpu_set_error(NRGPU_ERR_ARG, "queue mode %d (0, 1)", on);
   if (on >= 0) L->queue = on;
   return L->queue;
+}
+
+extern "C" int nrgpu_level_parts(nrgpu_level *L, int on) {
+  if (!L) return nrgpu_set_error(NRGPU_ERR_ARG, "null level");
+  if (on > 1) return nrgpu_set_error(NRGPU_ERR_ARG, "two-kernel mode %d (0, 1)", on);
+  if (on >= 0) L->parts = on;
+  return L->parts;
+}
+
+extern "C" int nrgpu_level_route(nrgpu_level *L, int system, const void *params, int box) {
+  if (!L || !params || box < 0 || box >= L->nboxes || (system != NRGPU_SYSTEM_BSSN && system != NRGPU_SYSTEM_Z4C))
+    return nrgpu_set_error(NRGPU_ERR_ARG, "bad route arguments");
+  int e;
+  if (system == NRGPU_SYSTEM_Z4C) {
+    const nrgpu_z4_params &p = *(const nrgpu_z4_params *)params;
+    if ((e = z4_check_params(&p))) return e;
+    return z4_route(L, L->step_work, nrgpu_rhs_run(L, p), box, p, true);
+  }
+  const nrgpu_bssn_params &p = *(const nrgpu_bssn_params *)params;
+  if ((e = check_params(&p))) return e;
+  const double *u[NRGPU_NV];
+  for (int v = 0; v < NRGPU_NV; ++v) u[v] = L->scratch + (long)v * L->npoints;
+  return bssn_route(L, L->step_work, nrgpu_rhs_run(L, p), box, u, p);
 }
 
 extern "C" int nrgpu_level_tile(nrgpu_level *L, int on) {

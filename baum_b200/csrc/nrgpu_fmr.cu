@@ -1006,6 +1006,12 @@ extern "C" int nrgpu_fmr_block(nrgpu_fmr *F, int l, int *block) {
   return nrgpu_level_get_block(F->L[l], block);
 }
 
+extern "C" int nrgpu_fmr_route(nrgpu_fmr *F, int l, int box) {
+  if (!F || l < 0 || l >= F->nl) return nrgpu_set_error(NRGPU_ERR_ARG, "no level %d", l);
+  return nrgpu_level_route(F->L[l], F->p.system,
+                           F->p.system == NRGPU_SYSTEM_BSSN ? (const void *)&F->bp[l] : (const void *)&F->zp[l], box);
+}
+
 extern "C" int nrgpu_fmr_iteration(nrgpu_fmr *F, int l) {
   if (!F || l < 0 || l >= F->nl) return -1;
   return F->iteration[l];

@@ -139,6 +139,14 @@ class Hierarchy:
         abi.check(abi.lib().nrgpu_fmr_block(self.handle, l, b))
         return tuple(b)
 
+    def route(self, l, box=0):
+        """The kernels of level l's interior rhs on a box, one of abi.ROUTES
+        (nrgpu_fmr_route)."""
+        r = abi.lib().nrgpu_fmr_route(self.handle, int(l), int(box))
+        if r < 0:
+            abi.check(r)
+        return abi.ROUTES[r]
+
     def save(self):
         """The hierarchy's own state (iteration counters, previous-step
         copies, time interpolants) as a numpy byte array (nrgpu_fmr_save)."""

@@ -356,6 +356,8 @@ int nrgpu_fmr_advance(nrgpu_fmr *fmr, double *const *u, int nsteps, void *stream
 int nrgpu_fmr_iteration(nrgpu_fmr *fmr, int l);
 /* the rhs block shape (x, y, z) level l runs with, into block[3] */
 int nrgpu_fmr_block(nrgpu_fmr *fmr, int l, int *block);
+/* the kernels of the interior rhs of box `box` of level l (nrgpu_level_route) */
+int nrgpu_fmr_route(nrgpu_fmr *fmr, int l, int box);
 
 /* Checkpoint of the hierarchy's own state (no counterpart: the reference's
  * checkpoint, main/main/checkpoint.c:14-165, writes the level variables,
@@ -525,6 +527,18 @@ enum { NRGPU_SYSTEM_BSSN = 0, NRGPU_SYSTEM_Z4C = 1 };
 int nrgpu_level_autotune(nrgpu_level *L, int system, const void *params, void *stream, int *best_block);
 int nrgpu_level_block(nrgpu_level *L, int bx, int by, int bz);
 int nrgpu_level_get_block(nrgpu_level *L, int *block);
+/* The two kernels on the boxes and runs they cover: on = 1 (the default of a
+ * level), 0 point by point, -1 only queries.  Returns the setting. */
+int nrgpu_level_parts(nrgpu_level *L, int on);
+/* Which kernels the next RK step of the level (nrgpu_bssn_rk4_step,
+ * nrgpu_z4_rk4_step) would run on the interior of box `box`, with the
+ * settings and the workspace that the level has (allocated by its first step
+ * or by nrgpu_level_autotune): one of NRGPU_ROUTE_*, or an error.  POINT: one
+ * thread per point, on the caller's lists; STAGED: the same on the staging
+ * copy; PARTS: the two kernels; TILE, QUEUE: below.  Rounding differences
+ * only between PARTS, TILE and the others, none among the others. */
+enum { NRGPU_ROUTE_POINT = 0, NRGPU_ROUTE_STAGED = 1, NRGPU_ROUTE_PARTS = 2, NRGPU_ROUTE_TILE = 3, NRGPU_ROUTE_QUEUE = 4 };
+int nrgpu_level_route(nrgpu_level *L, int system, const void *params, int box);
 /* The BSSN interior rhs over TMA-staged tiles on every box it covers (runs
  * of order 4 or 6, even row length, 16-byte aligned fields, advection shift
  * 1 or 2 at 4th order, the centred 6th-order advection), the per-point

@@ -77,21 +77,25 @@ def test_staged_box_matches_oracle(gpu, n_inner, order):
     (100^3 and 72^3 with the boundary layer: staged into copies with the
     strides of 104, and the 72 kernel itself at 6th order): the puncture
     box at dx = 0.25 with a shift, 2 RK4 steps, every variable within 1e-12
-    of the oracle."""
+    of the oracle; and the same by the two kernels."""
     lev, u0 = punctures.schwarzschild_c1(n_inner, 0.25)
     x, _, _ = lev.coords()
     u0[18] = 0.05 * np.sin(0.3 * x)
     p = abi.bssn_params(**(CASES["bssn_fourier_o6"] if order == 6 else {}))
     dt = 0.25 * 0.25
-    dl = bssn.DeviceLevel(lev)
-    u = to_dev(u0)
-    for _ in range(2):
-        bssn.evolve_rk_rk4(dl, u, dt, p)
-    torch.cuda.synchronize()
-    uo = oracle.bssn_evolve(lev, np.ascontiguousarray(u0), dt, 2, p)
-    err = relerr(u.cpu().numpy(), uo)
-    assert err.max() < TOL, err
-    assert not dl.nan_flag()
+    uo = oracle.bssn_evolve(lev, np.ascontiguousarray(u0.copy()), dt, 2, p)
+    for route in ("point" if n_inner == 70 else "staged", "parts"):
+        dl = bssn.DeviceLevel(lev)
+        dl.parts(int(route == "parts"))
+        u = to_dev(u0)
+        for _ in range(2):
+            bssn.evolve_rk_rk4(dl, u, dt, p)
+        torch.cuda.synchronize()
+        assert dl.route(p) == route
+        err = relerr(u.cpu().numpy(), uo)
+        assert err.max() < TOL, (route, err)
+        assert not dl.nan_flag()
+        dl.close()
 
 
 def test_c1_schwarzschild_50_steps_matches_oracle(gpu):

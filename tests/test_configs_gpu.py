@@ -5,11 +5,13 @@ benchmarked grids (162^3: the precision-sweep box and level 0 of the batched
 refinement grid; 168^3, 136^3, 104^3, 72^3: its finer levels; 194^3 and
 136^3 at 6th order: the levels of the full form's grid, 72^3 at 6th order its
 moving puncture boxes; 106^3 and 98^3: boxes of other sizes, staged into
-a copy with the strides of the next size).  Each instance is run here
-on a single box of its size through the C ABI and compared with the CPU
-oracle (1e-12 relative per variable, the bar of every rhs parity test): the
+a copy with the strides of the next size).  Each instance, and the
+two-kernel rhs that large boxes run outside deep hierarchies, is run here on a
+single box of its size through the C ABI and compared with the CPU oracle
+(1e-12 relative per variable, the bar of every rhs parity test): the
 precision-sweep box at its full size (160^3 inner points, 6th order) for
-two RK4 steps, the others for one.  The batched 7-level grid itself is
+two RK4 steps, the others for one.  The rhs of every instance of both systems,
+and of a staged box for it, is compared with the two kernels besides.  The batched 7-level grid itself is
 compared with the oracle at reduced size (the same uneven pattern of
 levels, every level stepped 2^l times per coarse step, restriction,
 prolongation and time interpolation in between), and at its full size
@@ -25,7 +27,7 @@ import pytest
 import torch
 
 from conftest import GOLDEN, relerr
-from baum_b200 import abi, fmr, punctures, workloads, z4
+from baum_b200 import abi, bssn, fmr, punctures, workloads, z4
 from oracle import oracle
 
 pytestmark = pytest.mark.gpu
@@ -53,20 +55,52 @@ def test_fixed_stride_instance_matches_oracle(gpu, m, order, steps):
     lev = abi.Level.single_box(m, dx)
     u0 = shifted_binary(lev, 5.0)
     p = abi.z4_params(order_centered=order, order_advection=order)
-    dl = z4.DeviceLevel(lev)
-    u = torch.from_numpy(u0.copy()).cuda()
     dt = 0.25 * dx
-    for _ in range(steps):
-        z4.evolve_rk_rk4(dl, u, dt, p)
-    torch.cuda.synchronize()
-    assert not dl.nan_flag()
-    got = u.cpu().numpy()
-    dl.close()
-    del u
-    torch.cuda.empty_cache()
-    uo = oracle.z4_evolve(lev, np.ascontiguousarray(u0), dt, steps, p)
-    err = relerr(got, uo)
-    assert err.max() < TOL, (m, order, err.max(), int(err.argmax()))
+    uo = oracle.z4_evolve(lev, np.ascontiguousarray(u0.copy()), dt, steps, p)
+    for route in ("staged" if m in (106, 98) else "point", "parts"):
+        dl = z4.DeviceLevel(lev)
+        dl.parts(int(route == "parts"))
+        u = torch.from_numpy(u0.copy()).cuda()
+        for _ in range(steps):
+            z4.evolve_rk_rk4(dl, u, dt, p)
+        torch.cuda.synchronize()
+        assert dl.route(p) == route
+        assert not dl.nan_flag()
+        err = relerr(u.cpu().numpy(), uo)
+        dl.close()
+        del u
+        torch.cuda.empty_cache()
+        assert err.max() < TOL, (m, order, route, err.max(), int(err.argmax()))
+
+
+@pytest.mark.parametrize("system", ["bssn", "z4"])
+@pytest.mark.parametrize("order", [4, 6])
+@pytest.mark.parametrize("m", [66, 72, 104, 136, 162, 168, 194])
+def test_point_instances_match_the_two_kernels(gpu, m, order, system):
+    """m x m x 30 (the instance of that size) and (m - 1) x (m - 3) x 30
+    (staged with its strides) point by point, and by the two kernels.  Both
+    are within 1e-12 of the exact rhs, so within twice that of each other."""
+    from test_parts_gpu import box, state
+    mod = bssn if system == "bssn" else z4
+    p = (abi.bssn_params if system == "bssn" else abi.z4_params)(order_centered=order, order_advection=order)
+    for shape, want in (((m, m, 30), "point"), ((m - 1, m - 3, 30), "staged")):
+        lev = box(*shape)
+        u0 = state(lev, system)
+        u = torch.from_numpy(u0).cuda()
+        out = []
+        for parts in (0, 1):
+            dl = mod.DeviceLevel(lev)
+            dl.parts(parts)
+            if parts == 0:
+                # the route is that of the steps: one, on a copy
+                mod.evolve_rk_rk4(dl, u.clone(), 0.01, p)
+                assert dl.route(p) == want
+            r = dl.empty(u0.shape[0])
+            mod.evolve_rhs(dl, r, u, 0.0, u, p)
+            out.append(r.cpu().numpy())
+            dl.close()
+        err = relerr(out[0], out[1])
+        assert 0 < err.max() < 2 * TOL, (shape, err.max(), int(err.argmax()))
 
 
 def test_seven_level_grid_matches_oracle(gpu):

@@ -213,3 +213,46 @@ def test_time_interpolation_orders_4_and_6(gpu, order, steps):
     for a, b in zip(saved, got):
         assert np.array_equal(a.cpu().numpy(), b)
     H2.close()
+
+
+@pytest.mark.parametrize("system", ["bssn", "z4"])
+def test_two_kernel_hierarchy_matches_oracle(gpu, system):
+    """Three levels large enough for the two-kernel rhs (48^3 to 52^3 inner
+    points): two coarse steps against the oracle, graph replay equal to plain
+    launches, and a hierarchy loaded from the checkpoint between the two, whose
+    first step is already replayed, equal to the run without it."""
+    levels = fmr.nested_levels([50, 52, 52], 0.5)
+    bssn = system == "bssn"
+    params = [(abi.bssn_params if bssn else abi.z4_params)(dissfactor=(0.1 if l == 0 else 0.02) / 64) for l in range(3)]
+    dt = [0.125 / 2 ** l for l in range(3)]
+    nv, unit = (abi.NVARS, synthetic.BSSN_UNIT) if bssn else (abi.Z4_NVARS, synthetic.Z4_UNIT)
+    u0 = []
+    for lev in levels:
+        x, y, z = lev.coords()
+        u0.append(synthetic.fourier_state(x, y, z, nv, unit, 8, 0.05, 16.0, 3))
+    fp = lambda g: abi.fmr_params(system=abi.SYSTEM_BSSN if bssn else abi.SYSTEM_Z4C, use_graph=g)  # noqa: E731
+    runs = []
+    for use_graph in (0, 1):
+        H = fmr.Hierarchy(levels, dt, params, fp(use_graph))
+        u = [to_dev(x) for x in u0]
+        H.advance(u, 1)
+        if use_graph:
+            buf, saved = H.save(), [x.clone() for x in u]
+        H.advance(u, 1)
+        torch.cuda.synchronize()
+        assert [H.route(l) for l in range(3)] == ["parts"] * 3
+        runs.append([x.cpu().numpy() for x in u])
+        H.close()
+    H = fmr.Hierarchy(levels, dt, params, fp(1))
+    H.load(buf)
+    H.advance(saved, 1)
+    torch.cuda.synchronize()
+    runs.append([x.cpu().numpy() for x in saved])
+    H.close()
+    for a, b, c in zip(*runs):
+        assert np.array_equal(a, b) and np.array_equal(a, c)
+    st = oracle.FmrState(levels, u0, 0 if bssn else 1, params, dt)
+    st.advance(2)
+    for l in range(3):
+        err = np.abs(runs[0][l] - st.u[l]).max(axis=1) / np.maximum(np.abs(st.u[l]).max(axis=1), 1e-8)
+        assert err.max() < FMR_TOL, (l, err.max())

@@ -229,3 +229,51 @@ def test_tuner_leaves_the_shape_where_the_two_kernels_run(gpu):
     assert dl.autotune(abi.SYSTEM_BSSN, abi.bssn_params()) == (4, 4, 8)
     assert dl.tile() == 0
     dl.close()
+
+
+def test_boxes_of_a_level_share_the_lists(gpu):
+    """Two boxes of different sizes on the two kernels and a third below their
+    size: two RK4 steps of each system against the oracle."""
+    shapes = [(60, 52, 44), (47, 43, 41), (30, 28, 26)]
+    one = [box(*s) for s in shapes]
+    boxes = []
+    for q, lv in enumerate(one):
+        b = lv.boxes[0]
+        boxes.append((b.m, b.n, b.o, b.x0 + 25.0 * (q - 1), b.y0, b.z0))
+    lev = abi.Level(boxes, 0.3, np.concatenate([lv.boundary for lv in one]))
+    for system, mod, p, evolve in (("bssn", bssn, abi.bssn_params(), oracle.bssn_evolve),
+                                   ("z4", z4, abi.z4_params(), oracle.z4_evolve)):
+        u0 = state(lev, system)
+        dl = mod.DeviceLevel(lev)
+        u = torch.from_numpy(u0.copy()).cuda()
+        for _ in range(2):
+            mod.evolve_rk_rk4(dl, u, 0.05, p)
+        torch.cuda.synchronize()
+        assert [dl.route(p, b) for b in range(3)] == ["parts", "parts", "staged"]
+        e = relerr(u.cpu().numpy(), evolve(lev, np.ascontiguousarray(u0), 0.05, 2, p))
+        assert e.max() < TOL, e
+        dl.close()
+
+
+@pytest.mark.parametrize("shape,over", [
+    ((66, 66, 66), {}), ((60, 52, 44), {}),
+    ((41, 63, 70), {"order_centered": 6, "order_advection": 6, "advection_lopsided6": 2}),
+])
+def test_host_buffer_steps_equal_device_steps(gpu, shape, over):
+    """evolve_host, whose first and last stages run the two kernels slab by slab
+    as copies of other slabs are on their way: one and three steps from pinned
+    memory, bit for bit those of the state on the device."""
+    lev = box(*shape)
+    p = abi.bssn_params(**over)
+    u0 = state(lev, "bssn")
+    for steps in (1, 3):
+        dl = bssn.DeviceLevel(lev)
+        u = torch.from_numpy(u0.copy()).cuda()
+        for _ in range(steps):
+            bssn.evolve_rk_rk4(dl, u, 0.05, p)
+        torch.cuda.synchronize()
+        assert dl.route(p) == "parts"
+        h = torch.from_numpy(u0.copy()).pin_memory()
+        bssn.evolve_host(dl, h, steps, 0.05, p)
+        assert torch.equal(h, u.cpu())
+        dl.close()

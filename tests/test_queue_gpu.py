@@ -3,7 +3,9 @@ boxes of a level in one persistent launch, the blocks taking tiles from an
 atomic counter.  Each point is computed by the same code as the per-box
 launch, so the rhs and the RK4 steps are bit-identical with the queue on and
 off: two and three 72^3 boxes (the full form's puncture boxes) at 4th and
-6th order, in the rhs, add-linear and RK4 epilogues."""
+6th order, in the rhs, add-linear and RK4 epilogues.  The queue takes the place
+of per-box launches point by point, so the two-kernel rhs is switched off, or
+the run is one that it does not cover."""
 import numpy as np
 import pytest
 import torch
@@ -31,15 +33,19 @@ def state(lev):
     return u
 
 
-@pytest.mark.parametrize("nboxes,order", [(2, 4), (3, 6), (2, 6)])
-def test_queue_kernel_is_identical_to_per_box_launches(gpu, nboxes, order):
+@pytest.mark.parametrize("nboxes,order,over", [(2, 4, {}), (3, 6, {}), (2, 6, {}),
+                                               (2, 4, {"advection_lopsided": 0})])
+def test_queue_kernel_is_identical_to_per_box_launches(gpu, nboxes, order, over):
     lev = boxes_level(nboxes)
     u0 = state(lev)
-    p = abi.z4_params(order_centered=order, order_advection=order)
+    p = abi.z4_params(order_centered=order, order_advection=order, **over)
     runs = []
     for on in (0, 1):
         dl = z4.DeviceLevel(lev)
+        if not over:
+            assert dl.parts(0) == 0
         assert dl.queue(on) == on
+        assert dl.route(p) == ("queue" if on else "point")
         u = torch.from_numpy(u0.copy()).cuda()
         r = dl.empty(25)
         z4.evolve_rhs(dl, r, u, 0.0, u, p)
@@ -67,7 +73,9 @@ def test_queue_needs_equal_boxes_of_a_kernel_size(gpu):
     out = []
     for on in (0, 1):
         dl = z4.DeviceLevel(lev)
+        dl.parts(0)
         dl.queue(on)
+        assert dl.route(p, 0) == dl.route(p, 1) == "point"
         u = torch.from_numpy(u0.copy()).cuda()
         z4.evolve_rk_rk4(dl, u, 0.05, p)
         torch.cuda.synchronize()
