@@ -892,6 +892,22 @@ extern "C" int nrgpu_fmr_create(int nl, const nrgpu_level_desc *levels, const do
   F->nl = nl;
   F->p = *p;
   F->nv = p->system == NRGPU_SYSTEM_BSSN ? NRGPU_NV : NRGPU_Z4_NVARS;
+  // The two-kernel rhs rounds its algebra in another order than the
+  // point-by-point kernels: after one coarse step the finest levels differ, of
+  // the state's norm, by about 2^-53 dt / dx^2, dt the coarse step and dx the
+  // finest spacing (a last bit of a field of unit background is a second
+  // difference of 2^-53 / dx^2, which acts for dt).  Measured over 3 to 8
+  // levels, coarse spacings 1/32 to 2 and both orders: 1e-16 to 3e-14 up to
+  // dt / dx^2 = 256; 3e-14 to 1.1e-13 at 512; 1.3e-13 at 1024, 2e-13 to 3e-13
+  // at 2048.  Both kernels are as far from a 64-bit evaluation as each other
+  // (3.7e-11 on level 6 of seven from dx 0.5, equal to three digits).  So that
+  // a run's results do not depend on its kernels by more than 1e-13 per coarse
+  // step, the two kernels run on hierarchies up to 4e-14 by this estimate,
+  // between 256 and 512, and the point-by-point kernels beyond (seven levels
+  // from 0.5: 787 ms per coarse step against 579).
+  double finest = 1e300;
+  for (int l = 0; l < nl; ++l) finest = fmin(finest, fmin(levels[l].dx, fmin(levels[l].dy, levels[l].dz)));
+  const bool parts = ldexp(dt[0], -53) <= NRGPU_PARTS_MAX_NOISE * finest * finest;
   int e = NRGPU_OK;
   for (int l = 0; l < nl && !e; ++l) {
     const nrgpu_level_desc &d = levels[l];
@@ -913,16 +929,7 @@ extern "C" int nrgpu_fmr_create(int nl, const nrgpu_level_desc *levels, const do
     if (p->system == NRGPU_SYSTEM_BSSN) F->bp[l] = ((const nrgpu_bssn_params *)sysparams)[l];
     else F->zp[l] = ((const nrgpu_z4_params *)sysparams)[l];
     if ((e = nrgpu_level_create(&d, &F->L[l]))) break;
-    // The two-kernel rhs rounds its algebra in another order than the
-    // point-by-point kernels.  Differences of a last bit in a field of unit
-    // background become second differences of 1e-16 / dx^2, and every level
-    // quarters dx^2 and doubles the substeps: after one coarse step the two
-    // differ, of the state's norm, by 1e-15 on level 3 (dx 1/16), 5e-15 on
-    // level 4, 6e-14 on level 5 and 3e-13 on level 6.  Hierarchies deeper than
-    // five levels keep the point-by-point kernels on every level, whose
-    // results then stay what they were to the last bit (seven levels: 787 ms
-    // per coarse step against 579).
-    F->L[l]->parts = nl <= NRGPU_PARTS_MAX_LEVELS;
+    F->L[l]->parts = parts;
     double *scr;
     if ((e = nrgpu_level_scratch(F->L[l], &scr))) break;  // no allocation later, inside a graph capture
     if (l > 0 && (e = setup_pair(F, l))) break;

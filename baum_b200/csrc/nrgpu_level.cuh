@@ -73,8 +73,8 @@ struct nrgpu_level {
   double *scratch;
   size_t scratch_points;
   // 1: the interior rhs by the two kernels of nrgpu_deriv.cuh where they
-  // cover the run; 0: point by point (the levels of a deep hierarchy,
-  // nrgpu_fmr_create)
+  // cover the run; 0: point by point (nrgpu_level_parts; the levels of a
+  // hierarchy of fine spacing, nrgpu_fmr_create)
   int parts;
   // step_work: of the RK steps, which no more overlap each other than they
   // may on the scratch.  call_work: of the rhs calls, which otherwise share
@@ -152,7 +152,7 @@ inline int nrgpu_pad_size(int m, int n) {
 #define NRGPU_DERIV_LISTS 71
 #define NRGPU_DERIV_PITCH 128
 #define NRGPU_PARTS_MIN_POINTS 50000
-#define NRGPU_PARTS_MAX_LEVELS 5
+#define NRGPU_PARTS_MAX_NOISE 4e-14
 // what a run's parameters allow on a level: the two kernels (FP64, advection
 // rows shifted by 1 or 2 (centred) at 4th order, by 2 or 3 (centred) at 6th; a
 // BSSN level whose staged tiles are switched on takes those), and a staging
@@ -176,9 +176,16 @@ inline RhsRun nrgpu_rhs_run(const nrgpu_level *L, const nrgpu_z4_params &p) {
           p.order_centered >= 4 && p.precision == 0};
 }
 // whether a run takes the two kernels on a box, given their lists: the one
-// rule of the launches, the allocation and the tuner.  Small boxes leave most
-// SMs idle either way, and one launch is cheaper than two: 34^3 step 217 us
-// point by point against 222, 50^3 774 against 563
+// rule of the launches, the allocation and the tuner.  The smallest boxes
+// leave most SMs idle either way, and then one launch costs what two do.  Step
+// point by point against the two kernels, in us, by inner points (cubes):
+//          27000    32768    39304    46656    54872    97336
+//   BSSN 4 225/225  380/250  412/245  464/320  475/324  720/510
+//   Z4c 4  236/224  404/248  439/270  505/310  522/326  786/536
+//   BSSN 6 352/330  582/333  629/381  672/395  758/440
+// The line at 50000 is on the safe side of the crossing near 30000, and stays
+// there although the boxes between would gain: they have their results to the
+// last bit from the point-by-point kernels.
 inline bool nrgpu_two_kernels(const RhsRun &run, const BoxGeo &b) {
   const int f = run.order;  // two faces of order / 2 points
   return run.two && b.m > f && b.n > f && b.o > f &&

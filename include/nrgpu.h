@@ -498,8 +498,10 @@ enum { NRGPU_SYSTEM_BSSN = 0, NRGPU_SYSTEM_Z4C = 1 };
 /* ---- launch-shape autotuner (no counterpart in the reference) -------------
  * Boxes of at least 50000 inner points run their 4th- and 6th-order interior
  * rhs in two kernels that choose their own tiles (advection shifts 1 and 2 at
- * 4th order, 2 and 3 at 6th; FP64; not on the levels of a hierarchy deeper
- * than five, nor where nrgpu_level_tile is on): where every box does, nothing is
+ * 4th order, 2 and 3 at 6th; FP64; not on the levels of a hierarchy whose
+ * coarse step dt and finest spacing dx have dt / dx^2 > 360, where the rounding
+ * of the two would differ by more than 1e-13 of the state per coarse step, nor
+ * on a BSSN level with nrgpu_level_tile on): where every box does, nothing is
  * timed and the level's shape stays, and where one does, neither staged tiles
  * nor the queue are tried.  Their
  * intermediate lists take up to 512 MB per level for the RK steps and as much

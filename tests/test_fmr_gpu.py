@@ -256,3 +256,15 @@ def test_two_kernel_hierarchy_matches_oracle(gpu, system):
     for l in range(3):
         err = np.abs(runs[0][l] - st.u[l]).max(axis=1) / np.maximum(np.abs(st.u[l]).max(axis=1), 1e-8)
         assert err.max() < FMR_TOL, (l, err.max())
+
+
+@pytest.mark.parametrize("nl,dx,route", [(5, 0.25, "parts"), (5, 0.125, "staged"), (6, 1.0, "parts"), (6, 0.5, "staged"),
+                                         (7, 4.0, "parts"), (3, 0.0125, "parts"), (3, 0.01, "staged")])
+def test_two_kernels_up_to_a_rounding_noise(gpu, nl, dx, route):
+    """The two-kernel rhs on hierarchies by what its rounding does to a coarse
+    step, 2^-53 dt / dx^2 with the finest dx, not by the number of levels."""
+    levels = fmr.nested_levels([46] + [44] * (nl - 1), dx)
+    dt = [0.25 * dx / 2 ** l for l in range(nl)]
+    H = fmr.Hierarchy(levels, dt, [abi.z4_params(dissfactor=0.02 / 64)] * nl)
+    assert [H.route(l) for l in range(nl)] == [route] * nl
+    H.close()
