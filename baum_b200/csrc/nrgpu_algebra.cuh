@@ -9,10 +9,8 @@
 // are contracted pairwise (the connection terms of the Ricci tensor through
 // one raised index: 216 products per point instead of 540; A~ A~ and A~^ij
 // through A~^i_j: 63 instead of 216).  Algebraically these are the
-// reference's expressions; only the rounding differs.  (Over the
-// 64 substeps of a seven-level hierarchy the refined fields amplify any
-// rounding difference to 3e-13 of the state's norm: there the levels keep the
-// point-by-point kernels, nrgpu_fmr_create.)
+// reference's expressions; only the rounding differs (which the levels of a
+// hierarchy of fine spacing amplify: nrgpu_fmr_create).
 //
 // A source S gives, at its point,
 //   val(v)               the variable
